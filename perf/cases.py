@@ -239,6 +239,77 @@ def run(s):
     return {"token": out["token"].to_u32(), "logits": _floats(out["logits"])}
 
 
+# ---- the same in 64 bits ---------------------------------------------------------------------------------------------
+
+def _act64(name, x):
+    if name == "GELU_TANH":
+        return 0.5 * x * (1.0 + torch.tanh(math.sqrt(2.0 / math.pi) * (x + 0.044715 * x ** 3)))
+    return {"NONE": lambda t: t, "RELU": torch.relu, "SILU": torch.nn.functional.silu, "GELU": torch.nn.functional.gelu}[name](x)
+
+
+def _linear64(x, w, bias=None, residual=None, act="NONE", gate=False, scale=1.0):
+    y = x.double() @ w.double().t()
+    if bias is not None:
+        y = y + bias.double()
+    if gate:
+        h = y.shape[-1] // 2
+        y = _act64(act, y[..., :h]) * y[..., h:]
+    else:
+        y = _act64(act, y)
+    y = y * scale
+    return y if residual is None else y + residual.double()
+
+
+def exact(case, seed):
+    """What run returns, in float64 from the stored operands (nothing between the layers is rounded); the operands are drawn
+    in the order in which the preparations above draw them."""
+    c, g = case, _gen(seed)
+    if c["kind"] == "linear":
+        M, K, N = c["M"], c["K"], c["N"]
+        w, b = _normal(g, (N, K), c["w"], 0.02), _normal(g, (N,), c["w"]) if c["bias"] else None
+        x, r = _normal(g, (M, K), c["io"]), _normal(g, (M, N // 2 if c["gate"] else N), c["io"]) if c["residual"] else None
+        return _linear64(x, w, b, r, c["act"], c["gate"])
+    if c["kind"] == "head":
+        scale, w = _normal(g, (c["K"],), "f32", 1.0), _normal(g, (c["N"], c["K"]), c["w"], 0.02)
+        torch.rand(1, generator=g, device="cuda")
+        x = _normal(g, (c["M"], c["K"]), "f32").double()
+        x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5) * scale.double()
+        return {"token": None, "logits": _linear64(x, w).cpu()}
+    p, M = presets.PRESETS[c["preset"]], c["M"]
+    specs = presets.block_linears(p)
+
+    def act_of(ex):
+        return p["act"] if ex.get("gate") or ex.get("act") else "NONE"
+
+    if c["kind"] == "block":
+        given = {name: (_normal(g, (N, K), c["w"], 0.02), _normal(g, (N,), c["w"], 0.02) if ex.get("bias") else None) for name, K, N, ex in specs}
+        hidden, attention, normed = (_normal(g, (M, n), c["io"]) for n in (p["d"], p["q"], p["d"]))
+        out = {}
+        for name, _, _, ex in specs:
+            w, b = given[name]
+            if name == "o":
+                out[name] = hidden = _linear64(attention, w, b, hidden)
+            elif name in ("down", "fc2"):
+                out[name] = _linear64(mid, w, b, hidden)
+            else:
+                out[name] = _linear64(normed, w, b, None, act_of(ex), bool(ex.get("gate")))
+                if name in ("gate_up", "fc1"):
+                    mid = out[name]
+        return out
+    given = [[(_normal(g, (N, K), c["w"], 0.02), _normal(g, (N,), c["w"], 0.02) if ex.get("bias") else None) for _, K, N, ex in specs]
+             for _ in range(c["layers"])]
+    head = _normal(g, (p["vocab"], p["d"]), c["w"], 0.02) if c["head"] else None
+    x = x0 = _normal(g, (M, p["d"]), c["io"]).double()
+    for layer in given:
+        made = {name: (w, b, act_of(ex), bool(ex.get("gate"))) for (name, _, _, ex), (w, b) in zip(specs, layer)}
+        attention = _linear64(x, *made["q"][:2]) if p["gated"] else x
+        h = _linear64(attention, *made["o"][:2], x0, scale=0.5)
+        w, b, act, gate = made["gate_up" if p["gated"] else "fc1"]
+        mid = _linear64(h, w, b, None, act, gate)
+        x = _linear64(mid, *made["down" if p["gated"] else "fc2"][:2], x0, scale=0.25)
+    return (x if head is None else _linear64(x, head)).cpu()
+
+
 # ---- what a pass cannot do without, and how far two correct ones may differ --------------------------------------------
 
 def _linear_work(M, K, N, io, w, bias, residual, gate):
