@@ -87,15 +87,20 @@ __host__ __device__ inline EpilogueArgs make_epilogue_args(const LinearArgs& a)
     return e;
 }
 
+// flat % elems; the 64-bit division only where the index needs it
+__device__ __forceinline__ size_t wrap_index(size_t flat, uint32_t elems)
+{
+    return flat >> 32 ? flat % elems : (size_t)((uint32_t)flat % elems);
+}
 __device__ __forceinline__ float read_bias(const EpilogueArgs& e, size_t flat)
 {
     if (!e.has_bias) return 0.0f;
-    return load_as_f32(e.bias, e.b_dtype, e.bias_elems ? flat % e.bias_elems : flat);
+    return load_as_f32(e.bias, e.b_dtype, e.bias_elems ? wrap_index(flat, e.bias_elems) : flat);
 }
 __device__ __forceinline__ float read_res(const EpilogueArgs& e, size_t flat)
 {
     if (!e.has_res) return 0.0f;
-    return load_as_f32(e.res, e.o_dtype, e.res_elems ? flat % e.res_elems : flat);
+    return load_as_f32(e.res, e.o_dtype, e.res_elems ? wrap_index(flat, e.res_elems) : flat);
 }
 
 // O = s*ep(acc + b) + R   or   s*ep(acc + b + R)   (vAi linear-slab.comp:236-241,
@@ -161,7 +166,21 @@ struct GemvArgmax {
 };
 
 // Launchers implemented in the .cu files; each returns a cudaError_t.
-struct GemvConfig { int rows_per_warp; int k_warps; int grid; size_t smem; int vectorized; int unroll; int plain_launch; };
+// Geometry of the streaming form (gemv_stream.cu): weight vectors per lane and row, warps that share a row's K, output
+// columns between two folds.
+struct GemvStream { int xv; uint32_t ks, batch; int grid; };
+// streaming: `stream` applies; else the register form's fields do.
+struct GemvConfig {
+    int rows_per_warp; int k_warps; int grid; size_t smem; int vectorized; int unroll; int plain_launch;
+    int streaming; GemvStream stream;
+};
+bool choose_gemv_stream(const LinearArgs& a, int sm_count, GemvStream* out);
+cudaError_t launch_gemv_stream(const LinearArgs& a, const GemvConfig& cfg, uint32_t nseg, const uint32_t* rows, const void* const* w,
+                               void* const* o, const GemvArgmax* argmax, cudaStream_t stream);
+constexpr uint32_t kSkinnyStreamRows = 8;
+// 1 <= M <= kSkinnyStreamRows, 16-bit weights, K % 8 == 0, I and W 16-byte aligned (skinny_stream.cu)
+cudaError_t launch_skinny_stream(const LinearArgs& a, int sm_count, uint32_t nseg, const uint32_t* rows, const void* const* w,
+                                 void* const* o, cudaStream_t stream);
 
 cudaError_t launch_gemv(const LinearArgs& a, const GemvConfig& cfg, cudaStream_t stream, const GemvArgmax* argmax = nullptr);
 // `tuning` (may be null) carries a caller's overrides of the geometry; see vaicu_linear_tuning.
@@ -257,7 +276,8 @@ cudaError_t launch_pdl_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, si
 struct SmemOptIn {
     static constexpr int kMaxDevices = 64;
     unsigned char done[kMaxDevices] = {};
-    template <typename Kernel> cudaError_t ensure(Kernel kern, int bytes)
+    // carveout: the share of an SM that shared memory should take, for kernels meant to share one (-1: the driver's choice)
+    template <typename Kernel> cudaError_t ensure(Kernel kern, int bytes, int carveout = -1)
     {
         int dev = -1;
         cudaError_t e = cudaGetDevice(&dev);
@@ -265,6 +285,7 @@ struct SmemOptIn {
         const bool tracked = dev >= 0 && dev < kMaxDevices;
         if (tracked && done[dev]) return cudaSuccess;
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess && carveout >= 0) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
         if (e == cudaSuccess && tracked) done[dev] = 1;
         return e;
     }

@@ -12,6 +12,8 @@
 //   * K is split over `k_warps` warps of a block when N alone cannot fill
 //     148 SMs; the fold goes through shared memory, no global scratch;
 //   * blocks are persistent over row groups (grid sized to the SM count).
+// Up to 4 rows whose activations fit the lanes' registers take the streaming form (gemv_stream.cu); this one keeps
+// longer K, 5 to 8 rows without tensor cores, and every geometry that a caller chooses.
 #include "common.cuh"
 
 namespace vaicu {
@@ -557,6 +559,12 @@ GemvConfig choose_gemv(const LinearArgs& a, int sm_count, bool ptrs_aligned16, c
     const int vec = a.w_dtype == VAICU_DTYPE_F32 ? 4 : 8;
     const uint32_t H = a.gate_fuse ? a.N / 2u : a.N;
     c.vectorized = ptrs_aligned16 && (a.K % (uint32_t)vec == 0u) && a.M >= 1u && a.M <= 8u;
+    const bool tuned = tuning && (tuning->gemv_rows || tuning->gemv_k_warps || tuning->gemv_unroll || tuning->gemv_grid || tuning->gemv_plain_launch);
+    if (c.vectorized && !tuned && choose_gemv_stream(a, sm_count, &c.stream)) {
+        c.streaming = 1;
+        c.grid = c.stream.grid;
+        return c;
+    }
     if (!c.vectorized) {
         c.rows_per_warp = 1; c.k_warps = 1; c.smem = 0;
         c.grid = (int)((H + kWarps - 1u) / kWarps);
@@ -639,6 +647,7 @@ cudaError_t launch_gemv_group(const LinearArgs& a, const GemvConfig& cfg, uint32
                               const void* const* w, void* const* o, cudaStream_t stream)
 {
     if (nseg < 2u || nseg > 3u || !cfg.vectorized || a.gate_fuse) return cudaErrorInvalidValue;
+    if (cfg.streaming) return launch_gemv_stream(a, cfg, nseg, rows, w, o, nullptr, stream);
     GemvParams p{};
     p.a = a;
     p.H = a.N;
@@ -671,11 +680,12 @@ cudaError_t launch_gemv_group(const LinearArgs& a, const GemvConfig& cfg, uint32
 
 cudaError_t launch_gemv(const LinearArgs& a, const GemvConfig& cfg, cudaStream_t stream, const GemvArgmax* argmax)
 {
+    if (argmax && (!cfg.vectorized || a.gate_fuse)) return cudaErrorInvalidValue;
+    if (cfg.streaming) return launch_gemv_stream(a, cfg, 0u, nullptr, nullptr, nullptr, argmax, stream);
     GemvParams p{};
     p.a = a;
     p.H = a.gate_fuse ? a.N / 2u : a.N;
     if (argmax) {
-        if (!cfg.vectorized || a.gate_fuse) return cudaErrorInvalidValue;
         p.am = *argmax;
     }
     if (!cfg.vectorized) {
