@@ -1,4 +1,5 @@
-"""The streaming decode form (gemv_stream.cu, up to 4 rows) at the sizes where its geometry can go wrong: K that fills no vector round, one that needs several warps or several register
+"""The streaming decode form (gemv_stream.cu for up to 4 rows, skinny_stream.cu for 5 to 8 on the tensor cores) at the
+sizes where its geometry can go wrong: K that fills no vector round, one that needs several warps or several register
 loads of activations, fewer columns than blocks, ranges that end inside a stage, more columns than one fold holds."""
 import numpy as np
 import pytest
@@ -17,20 +18,20 @@ def _draw(M, K, N, residual=True):
             rng.standard_normal(N).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32) if residual else None)
 
 
-@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 5, 8])
 @pytest.mark.parametrize("K,N", [(8, 3), (200, 147), (520, 149), (768, 768), (1032, 300), (2560, 611), (4096, 160), (4104, 152),
                                  (8192, 320), (12288, 150), (64, 70001)])
 @pytest.mark.parametrize("dt", [("f32", "f16", "f32"), ("bf16", "bf16", "bf16")])
 def test_streaming_plain(M, K, N, dt, device):
     x, w, b, r = _draw(M, K, N)
     got, want, node = run_linear(x, w, b, r, i_dtype=dt[0], w_dtype=dt[1], o_dtype=dt[2], epilogue="GELU", scalar_scale=0.5)
-    assert node.info.kernel == nodes.KERNEL_GEMV
+    assert node.info.kernel == (nodes.KERNEL_GEMV if M <= 4 else nodes.KERNEL_TC_SKINNY)
     assert node.info.launches == 1
     # fp32 sums; the error-function polynomial of the GELU is good to 1.5e-7 of its argument
     assert_close(got, want, out_tol(dt[2]), f"{M}x{K}x{N} {dt}")
 
 
-@pytest.mark.parametrize("M", [1, 3, 4])
+@pytest.mark.parametrize("M", [1, 3, 4, 6])
 @pytest.mark.parametrize("K,H", [(8, 5), (768, 1500), (2048, 149), (8192, 75), (520, 20000)])
 @pytest.mark.parametrize("w_dtype", ["bf16", "f16"])
 def test_streaming_gate(M, K, H, w_dtype, device):
@@ -39,7 +40,7 @@ def test_streaming_gate(M, K, H, w_dtype, device):
     assert_close(got, want, (1e-4, 1e-5), f"gate {M}x{K}x{H} {w_dtype}")
 
 
-@pytest.mark.parametrize("M", [1, 4])
+@pytest.mark.parametrize("M", [1, 4, 8])
 @pytest.mark.parametrize("K,widths", [(768, (128, 256, 128)), (2560, (2048, 1024, 1024)), (520, (128, 128))])
 def test_streaming_group(M, K, widths, device):
     """Sibling Linears of one input in one launch: ranges and stages that straddle the members."""
@@ -55,8 +56,9 @@ def test_streaming_group(M, K, widths, device):
     out = net(Tensor.from_numpy(x))
     assert next(iter(net._recordings.values())).kernel_launches == 1
     net.pool.check_guards()
+    xs = x if M <= 4 else seen(x, Dtype.BF16)
     for i, w in enumerate(ws):
-        assert_close(out[f"y{i}"].to_numpy(), orc.linear_f64(x, seen(w, Dtype.BF16)), (1e-4, 1e-5), f"member {i}")
+        assert_close(out[f"y{i}"].to_numpy(), orc.linear_f64(xs, seen(w, Dtype.BF16)), (1e-4, 1e-5), f"member {i}")
 
 
 @pytest.mark.parametrize("M", [1, 2, 4])
@@ -79,7 +81,7 @@ def test_streaming_argmax(M, N, device):
 
 def test_streaming_epilogues_and_orders(device):
     x, w, b, r = _draw(7, 776, 333)
-    for M in (2, 4):
+    for M in (2, 7):
         for ep in Epilogue:
             got, want, _ = run_linear(x[:M].copy(), w, b, r[:M].copy(), w_dtype="bf16", epilogue=ep.name,
                                       residual_order="BEFORE_EPILOGUE", scalar_scale=0.25)

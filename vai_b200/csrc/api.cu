@@ -111,6 +111,7 @@ struct vaicu_linear_plan {
     int kernel;               // VAICU_KERNEL_*
     // GEMV
     GemvConfig gemv_vec, gemv_any;
+    bool skinny_stream;        // M <= 8 on the tensor cores: plain calls take skinny_stream_kernel
     // FMA tile (also the fallback of the tensor-core plans)
     FmaTileConfig fma;
     bool fma_partial;
@@ -474,6 +475,12 @@ int validate_tuning(const vaicu_linear_tuning& t)
     return VAICU_OK;
 }
 
+// Whether the caller shapes the tcgen05 kernel.
+bool tunes_tc(const vaicu_linear_tuning& t)
+{
+    return t.tc_pair >= 0 || t.tc_wide >= 0 || t.tc_bn || t.tc_splits || t.tc_fold || t.tc_stages || t.tc_tile_rows || t.tc_tail_strips;
+}
+
 int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_linear_tuning& tuning, vaicu_linear_plan** out)
 {
     if (!dev || !out) return VAICU_ERR_INVALID_VALUE;
@@ -498,7 +505,7 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
     pl->gemv_vec = choose_gemv(a, dev->sm_count, true, &pl->tune);
     pl->gemv_any = choose_gemv(a, dev->sm_count, false, &pl->tune);
     plan_fma(pl);
-    pl->tc = false;
+    pl->tc = pl->skinny_stream = false;
     int kernel = force_kernel;
     if (kernel == 0) {
         // Few rows: the weight-streaming kernel (vAi useSlabPath takes M <= 8,
@@ -541,6 +548,10 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
             }
         }
         pl->launches = 1u + (pl->tc_cast ? 1u : 0u) + ((pl->tcp.splits > 1u && !pl->tile_done && !pl->tcp.cfold) ? 1u : 0u);
+        // Up to 8 rows the streaming form with mma.sync takes a plain call in one launch; a chosen kernel, a K span or
+        // any tuning of the tcgen05 kernel, outputs in several places and unaligned activations stay with that one.
+        pl->skinny_stream = kernel == VAICU_KERNEL_TC_SKINNY && force_kernel == 0 && d.M <= kSkinnyStreamRows && !d.split_size && !tunes_tc(tuning);
+        if (pl->skinny_stream) pl->launches = 1u;
         break;
     default:
         delete pl;
@@ -1073,6 +1084,10 @@ int run_impl(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const 
     }
     pl->last_kernel = pl->kernel;
     pl->last_vectorized = 1;
+    if (pl->skinny_stream && !spec && aligned16(I)) {
+        VAICU_CUDA(launch_skinny_stream(a, pl->dev->sm_count, 0u, nullptr, nullptr, nullptr, s));
+        return VAICU_OK;
+    }
     uint8_t* ws = reinterpret_cast<uint8_t*>(workspace);
     const void* act = I;
     if (pl->tc_cast) {
@@ -1280,8 +1295,19 @@ int vaicu_linear_run_group(vaicu_linear_plan* const* plans, int count, vaicu_str
         return VAICU_OK;
     }
     // swapped tensor-core kernel: one launch leaves the partial sums of all members, one fold stores the outputs
-    for (int i = 0; i < count; ++i)
+    bool one_launch = p0->kernel == VAICU_KERNEL_TC_SKINNY && aligned16(I);
+    for (int i = 0; i < count; ++i) {
         if (!aligned16(O[i])) return VAICU_ERR_UNSUPPORTED;
+        one_launch = one_launch && plans[i]->skinny_stream;
+    }
+    if (one_launch) {
+        vaicu_linear_desc all = p0->d;
+        all.N = (uint32_t)total;
+        const LinearArgs a = make_args(all, I, W[0], nullptr, nullptr, O[0]);
+        VAICU_CUDA(launch_skinny_stream(a, p0->dev->sm_count, (uint32_t)count, rows, W, O, s));
+        for (int i = 0; i < count; ++i) { plans[i]->last_kernel = VAICU_KERNEL_TC_SKINNY; plans[i]->last_vectorized = 1; }
+        return VAICU_OK;
+    }
     GroupState* g = nullptr;
     rc = group_state(plans, count, &g);
     if (rc != VAICU_OK) return rc;
