@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(kRmsThreads) row_norm_kernel(const RmsParams p
     __shared__ float s_part[kRmsThreads / 32];
     __shared__ float s_part2[kRmsThreads / 32];
     __shared__ float s_inv, s_mean;
+    launch_dependents();
+    dependency_wait();
     for (uint32_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
         const size_t base = (size_t)row * p.feat;
         float cache[kRmsCache];
@@ -102,8 +104,7 @@ cudaError_t launch_rms_norm(const void* in, const void* scale, const void* shift
     uint32_t grid = rows;
     const uint32_t cap = (uint32_t)sm_count * 8u;
     if (grid > cap) grid = cap;
-    row_norm_kernel<false><<<grid, kRmsThreads, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(row_norm_kernel<false>, dim3(grid), dim3(kRmsThreads), 0, stream, p);
 }
 
 cudaError_t launch_layer_norm(const void* in, const void* scale, const void* shift, const void* res, void* out, uint32_t rows,
@@ -113,8 +114,7 @@ cudaError_t launch_layer_norm(const void* in, const void* scale, const void* shi
     uint32_t grid = rows;
     const uint32_t cap = (uint32_t)sm_count * 8u;
     if (grid > cap) grid = cap;
-    row_norm_kernel<true><<<grid, kRmsThreads, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_pdl(row_norm_kernel<true>, dim3(grid), dim3(kRmsThreads), 0, stream, p);
 }
 
 }  // namespace vaicu

@@ -5,30 +5,48 @@
 // ascending); Z and the running sum accumulated in that order in fp32 with the row maximum
 // subtracted; the first rank whose running sum reaches u * Z is the sample (rank 0 if none).
 //
-// Two launches, as in the reference; the selection itself is organised for warps instead of
-// workgroup-wide rounds.  Stage 1: block (g, row) owns a 2048-column slice; each of its 8 warps
-// keeps 256 columns in registers (8 per lane, each lane's list sorted descending) and pops its
-// own top-k in k rounds of a warp-shuffle "best head" reduction (no block barrier), leaving a
-// sorted list in shared memory; warp 0 then merges the 8 sorted lists into the slice's top-k.
-// Stage 2: one warp merges the G sorted candidate lists (heads in registers, lists in shared
-// memory) and lane 0 samples.  Rows of at most 2048 columns need stage 1's block only.  Both
-// merges are exact: the top-k of a union is within the union of the parts' top-k.  u lives in
-// device memory so that a recorded launch sees each step's value.
+// Two launches, as in the reference.  Popping the best k times costs k dependent rounds of shuffles, so both
+// stages select by rank instead: a lower bound T on the k-th best is cheap (the k-th best of a few hundred maxima), few
+// entries reach it, and each of those counts how many outrank it - its place.
+// Stage 1: block (g, row) owns a 2048-column slice, 8 columns per thread; T is the k-th best of the 256 threads' maxima,
+// at most 8 k columns reach it.  Stage 2: T is the k-th best of the first ceil(k / G) entries of the G sorted lists.
+// Where more than 1024 entries reach that T (the winners crowd in a few slices) one warp merges the sorted lists.
+// Rows of at most 2048 columns need stage 1's block only.  Both steps are exact: the top-k of a union is within
+// the union of the parts' top-k.  u lives in device memory so that a recorded launch sees each step's value.
 #include "common.cuh"
 
 namespace vaicu {
 
 namespace {
 
-constexpr uint32_t kList = 8;             // register list length per thread
+constexpr uint32_t kList = 8;             // columns per thread
 constexpr uint32_t kMaxK = 128;           // vAi TopKSampling::maxK
 constexpr uint32_t kPartThreads = 256;    // stage 1: 256 * 8 = 2048 columns per block
 constexpr uint32_t kSlice = kPartThreads * kList;
+constexpr uint32_t kMaxKept = kMaxK * kList;   // entries that can reach stage 1's bound; stage 2's limit
 constexpr float kLowest = -3.4028235e38f; // the shader's sentinel (finite: softmax terms stay NaN-free)
 
 __device__ __forceinline__ bool outranks(float av, uint32_t ai, float bv, uint32_t bi)
 {
     return av > bv || (av == bv && ai < bi);
+}
+
+// The same order as one integer: larger is better.  NaN and what is below the sentinel rank with it (never chosen).
+typedef unsigned long long Key;
+constexpr Key kNone = 0;
+__device__ __forceinline__ Key rank_key(float v, uint32_t i)
+{
+    if (!outranks(v, i, kLowest, 0xFFFFFFFFu)) return kNone;
+    const uint32_t b = __float_as_uint(v + 0.0f);                  // -0 and +0 are equal: the index decides
+    return ((Key)(b & 0x80000000u ? ~b : b | 0x80000000u) << 32) | (Key)(~i);
+}
+// Entries of list[0, n) that outrank key.
+__device__ __forceinline__ uint32_t count_above(const Key* list, uint32_t n, Key key)
+{
+    uint32_t c = 0;
+#pragma unroll 8
+    for (uint32_t i = 0; i < n; ++i) c += list[i] > key ? 1u : 0u;
+    return c;
 }
 
 struct TopkParams {
@@ -102,20 +120,50 @@ __device__ __forceinline__ void merge_lists(const uint2* lists, uint32_t nlists,
     __syncwarp();
 }
 
-// Temperature softmax over the k winners and the inverse-CDF sample (topk-sampling.comp:237-258).
-__device__ __forceinline__ uint32_t sample(const float* top_v, const uint32_t* top_i, uint32_t k, float temperature, float u)
+// Temperature softmax over the k winners and the inverse-CDF sample (topk-sampling.comp:237-258).  Called by all
+// threads of a block; the exponentials are taken side by side (into `terms`), the sums run in rank order.
+__device__ __forceinline__ void sample(const float* top_v, const uint32_t* top_i, float* terms, uint32_t k, float temperature, float u,
+                                       uint32_t* out)
 {
     const float inv_t = 1.0f / fmaxf(temperature, 1e-6f);
     const float m = top_v[0];
+    for (uint32_t r = threadIdx.x; r < k; r += blockDim.x) terms[r] = expf((top_v[r] - m) * inv_t);
+    __syncthreads();
+    if (threadIdx.x != 0u) return;
     float z = 0.0f;
-    for (uint32_t r = 0; r < k; ++r) z += expf((top_v[r] - m) * inv_t);
+    for (uint32_t r = 0; r < k; ++r) z += terms[r];
     const float target = u * z;
     float cum = 0.0f;
+    uint32_t pick = top_i[0];
     for (uint32_t r = 0; r < k; ++r) {
-        cum += expf((top_v[r] - m) * inv_t);
-        if (cum >= target) return top_i[r];
+        cum += terms[r];
+        if (cum >= target) { pick = top_i[r]; break; }
     }
-    return top_i[0];
+    *out = pick;
+}
+
+// What the block keeps while it selects.
+struct Kept {
+    Key key[kMaxKept];
+    float val[kMaxKept];
+    Key best[kPartThreads];
+    float top_v[kMaxK];
+    uint32_t top_i[kMaxK];
+    float terms[kMaxK];
+    Key bound;
+    uint32_t count;
+};
+
+// The kept entries in rank order, the tail filled with sentinels.  All threads.
+__device__ __forceinline__ void place_by_rank(Kept& s, uint32_t count, uint32_t k)
+{
+    for (uint32_t c = threadIdx.x; c < count; c += kPartThreads) {
+        const Key key = s.key[c];
+        const uint32_t r = count_above(s.key, count, key);
+        if (r < k) { s.top_v[r] = s.val[c]; s.top_i[r] = ~(uint32_t)key; }
+    }
+    for (uint32_t r = count + threadIdx.x; r < k; r += kPartThreads) { s.top_v[r] = kLowest; s.top_i[r] = 0xFFFFFFFFu; }
+    __syncthreads();
 }
 
 // Stage 1.  SAMPLE: the row fits one block, which also samples.
@@ -123,91 +171,95 @@ template <bool SAMPLE>
 __global__ void __launch_bounds__(kPartThreads) topk_slice_kernel(const TopkParams p)
 {
     const uint32_t row = blockIdx.y, g = blockIdx.x, G = gridDim.x, tid = threadIdx.x;
-    const uint32_t warp = tid >> 5, lane = tid & 31u;
-    constexpr uint32_t kWarps = kPartThreads / 32u;
-    __shared__ uint2 warp_list[kWarps * kMaxK];          // each warp's top-k, descending
-    __shared__ float top_v[kMaxK];
-    __shared__ uint32_t top_i[kMaxK];
-
-    float lv[kList];
-    uint32_t li[kList];
-#pragma unroll
-    for (uint32_t j = 0; j < kList; ++j) { lv[j] = kLowest; li[j] = 0xFFFFFFFFu; }
+    __shared__ Kept s;
+    launch_dependents();
+    dependency_wait();
     const uint32_t slice = (p.N + G - 1u) / G;
     const uint32_t s0 = g * slice, s1 = (s0 + slice < p.N) ? s0 + slice : p.N;
-    for (uint32_t i = s0 + tid; i < s1; i += kPartThreads) {
-        const float v = load_as_f32(p.logits, p.dtype, (size_t)row * p.ld + i);
-        const uint32_t gi = p.index_base + i;
-        // insertion into the descending list (fully unrolled: the list stays in registers)
-        if (outranks(v, gi, lv[kList - 1], li[kList - 1])) {
-            lv[kList - 1] = v; li[kList - 1] = gi;
+    float v[kList];
+    Key key[kList], best = kNone;
 #pragma unroll
-            for (int q = kList - 1; q > 0; --q) {
-                if (outranks(lv[q], li[q], lv[q - 1], li[q - 1])) {
-                    const float tv = lv[q]; lv[q] = lv[q - 1]; lv[q - 1] = tv;
-                    const uint32_t ti = li[q]; li[q] = li[q - 1]; li[q - 1] = ti;
-                }
-            }
-        }
+    for (uint32_t j = 0; j < kList; ++j) {
+        const uint32_t i = s0 + tid + j * kPartThreads;
+        v[j] = i < s1 ? load_as_f32(p.logits, p.dtype, (size_t)row * p.ld + i) : kLowest;
     }
-    // k rounds inside the warp: the best list head wins and its lane pops
-    uint2* mine = warp_list + warp * p.k;
-    for (uint32_t r = 0; r < p.k; ++r) {
-        float bv = lv[0];
-        uint32_t bi = li[0];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
-            const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
-            if (outranks(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-        }
-        if (lane == 0u) mine[r] = make_uint2(__float_as_uint(bv), bi);
-        if (li[0] == bi && lv[0] == bv && bi != 0xFFFFFFFFu) {
-#pragma unroll
-            for (uint32_t q = 0; q + 1u < kList; ++q) { lv[q] = lv[q + 1]; li[q] = li[q + 1]; }
-            lv[kList - 1] = kLowest; li[kList - 1] = 0xFFFFFFFFu;
-        }
+    for (uint32_t j = 0; j < kList; ++j) {
+        const uint32_t i = s0 + tid + j * kPartThreads;
+        key[j] = i < s1 ? rank_key(v[j], p.index_base + i) : kNone;
+        best = key[j] > best ? key[j] : best;
     }
+    s.best[tid] = best;
+    if (tid == 0u) { s.bound = kNone; s.count = 0u; }
     __syncthreads();
-    if (warp != 0u) return;
-    merge_lists<1>(warp_list, kWarps, p.k, p.k, p.k, top_v, top_i, lane);
+    // keys of columns differ, so at most one thread is k-th; with fewer than k threads that hold any, all entries are kept
+    if (best != kNone && count_above(s.best, kPartThreads, best) == p.k - 1u) s.bound = best;
+    __syncthreads();
+    const Key bound = s.bound;
+#pragma unroll
+    for (uint32_t j = 0; j < kList; ++j)
+        if (key[j] != kNone && key[j] >= bound) {
+            const uint32_t at = atomicAdd(&s.count, 1u);
+            s.key[at] = key[j];
+            s.val[at] = v[j];
+        }
+    __syncthreads();
+    place_by_rank(s, s.count, p.k);
     if (SAMPLE) {
-        if (lane == 0u) p.out[row] = sample(top_v, top_i, p.k, p.temperature, *p.u);
+        sample(s.top_v, s.top_i, s.terms, p.k, p.temperature, *p.u, p.out + row);
     } else if (p.list_out) {
         // the row fits this block and its sorted list is the result: k entries, then padding
-        for (uint32_t r = lane; r < p.k_out; r += 32u)
-            p.list_out[(size_t)row * p.k_out + r] = r < p.k ? make_uint2(__float_as_uint(top_v[r]), top_i[r])
+        for (uint32_t r = tid; r < p.k_out; r += kPartThreads)
+            p.list_out[(size_t)row * p.k_out + r] = r < p.k ? make_uint2(__float_as_uint(s.top_v[r]), s.top_i[r])
                                                            : make_uint2(__float_as_uint(kLowest), 0xFFFFFFFFu);
     } else {
-        for (uint32_t r = lane; r < p.k; r += 32u)
-            p.cand_out[((size_t)row * G + g) * p.k + r] = make_uint2(__float_as_uint(top_v[r]), top_i[r]);
+        for (uint32_t r = tid; r < p.k; r += kPartThreads)
+            p.cand_out[((size_t)row * G + g) * p.k + r] = make_uint2(__float_as_uint(s.top_v[r]), s.top_i[r]);
     }
 }
 
-// Stage 2: one warp per row merges the G sorted lists (copied to shared memory when they fit).
-__global__ void __launch_bounds__(32) topk_merge_kernel(const TopkParams p, uint32_t lists_in_smem)
+// Stage 2: one block per row over its G <= 256 sorted lists.
+__global__ void __launch_bounds__(kPartThreads) topk_merge_kernel(const TopkParams p)
 {
-    extern __shared__ uint2 staged[];
-    __shared__ float top_v[kMaxK];
-    __shared__ uint32_t top_i[kMaxK];
-    const uint32_t row = blockIdx.x, lane = threadIdx.x, G = p.N;
+    const uint32_t row = blockIdx.x, tid = threadIdx.x, G = p.N;
+    __shared__ Kept s;
+    launch_dependents();
+    dependency_wait();
     const uint2* lists = p.cand_in + (size_t)row * p.row_stride;
-    size_t stride = p.list_stride;
-    if (lists_in_smem) {
-        for (uint32_t i = lane; i < G * p.list_len; i += 32u) staged[i] = lists[(size_t)(i / p.list_len) * stride + i % p.list_len];
-        __syncwarp();
-        lists = staged;
-        stride = p.list_len;
+    // the bound: the first entries of the lists, k of them where the lists are that long, at most 256: one per thread
+    const uint32_t even = (p.k + G - 1u) / G, ahead = even < p.list_len ? even : p.list_len;
+    Key mine = kNone;
+    if (tid < G * ahead) {
+        const uint2 c = lists[(size_t)(tid / ahead) * p.list_stride + tid % ahead];
+        mine = rank_key(__uint_as_float(c.x), c.y);
     }
-    if (G <= 64u) merge_lists<2>(lists, G, stride, p.list_len, p.k, top_v, top_i, lane);
-    else if (G <= 128u) merge_lists<4>(lists, G, stride, p.list_len, p.k, top_v, top_i, lane);
-    else merge_lists<8>(lists, G, stride, p.list_len, p.k, top_v, top_i, lane);
+    s.best[tid] = mine;
+    if (tid == 0u) { s.bound = kNone; s.count = 0u; }
+    __syncthreads();
+    if (mine != kNone && count_above(s.best, kPartThreads, mine) == p.k - 1u) s.bound = mine;
+    __syncthreads();
+    const Key bound = s.bound;
+    for (uint32_t i = tid; i < G * p.list_len; i += kPartThreads) {
+        const uint2 c = lists[(size_t)(i / p.list_len) * p.list_stride + i % p.list_len];
+        const Key key = rank_key(__uint_as_float(c.x), c.y);
+        if (key != kNone && key >= bound) {
+            const uint32_t at = atomicAdd(&s.count, 1u);
+            if (at < kMaxKept) { s.key[at] = key; s.val[at] = __uint_as_float(c.x); }
+        }
+    }
+    __syncthreads();
+    if (s.count <= kMaxKept) {
+        place_by_rank(s, s.count, p.k);
+    } else {
+        if (tid < 32u) merge_lists<8>(lists, G, p.list_stride, p.list_len, p.k, s.top_v, s.top_i, tid);
+        __syncthreads();
+    }
     if (p.list_out) {
-        for (uint32_t r = lane; r < p.k_out; r += 32u)
-            p.list_out[(size_t)row * p.k_out + r] = r < p.k ? make_uint2(__float_as_uint(top_v[r]), top_i[r])
+        for (uint32_t r = tid; r < p.k_out; r += kPartThreads)
+            p.list_out[(size_t)row * p.k_out + r] = r < p.k ? make_uint2(__float_as_uint(s.top_v[r]), s.top_i[r])
                                                            : make_uint2(__float_as_uint(kLowest), 0xFFFFFFFFu);
-    } else if (lane == 0u) {
-        p.out[row] = sample(top_v, top_i, p.k, p.temperature, *p.u);
+    } else {
+        sample(s.top_v, s.top_i, s.terms, p.k, p.temperature, *p.u, p.out + row);
     }
 }
 
@@ -217,17 +269,10 @@ __global__ void __launch_bounds__(32) topk_merge_kernel(const TopkParams p, uint
 uint32_t topk_groups(uint32_t N) { return (N + kSlice - 1u) / kSlice; }
 
 namespace {
-// Stage 2 over `G` lists per row; samples into `out`, or writes the merged list to `list_out`.
-cudaError_t launch_merge(const TopkParams& q, uint32_t M, uint32_t G, cudaStream_t stream)
+// Stage 2 over the lists of each row; samples into `out`, or writes the merged list to `list_out`.
+cudaError_t launch_merge(const TopkParams& q, uint32_t M, cudaStream_t stream)
 {
-    const size_t bytes = (size_t)G * q.list_len * sizeof(uint2);
-    const bool in_smem = bytes <= 200u * 1024u;
-    if (in_smem && bytes > 48u * 1024u) {
-        static SmemOptIn optin;
-        if (cudaError_t e = optin.ensure(topk_merge_kernel, (int)(200u * 1024u)); e != cudaSuccess) return e;
-    }
-    topk_merge_kernel<<<M, 32, in_smem ? bytes : 0, stream>>>(q, in_smem ? 1u : 0u);
-    return cudaGetLastError();
+    return launch_pdl(topk_merge_kernel, dim3(M), dim3(kPartThreads), 0, stream, q);
 }
 }  // namespace
 
@@ -246,14 +291,12 @@ cudaError_t launch_topk(const void* logits, int dtype, uint32_t M, uint32_t N, s
     p.k_out = K;
     const uint32_t G = topk_groups(N);
     if (G == 1u) {
-        if (list_out) topk_slice_kernel<false><<<dim3(1, M), kPartThreads, 0, stream>>>(p);
-        else topk_slice_kernel<true><<<dim3(1, M), kPartThreads, 0, stream>>>(p);
-        return cudaGetLastError();
+        return list_out ? launch_pdl(topk_slice_kernel<false>, dim3(1, M), dim3(kPartThreads), 0, stream, p)
+                        : launch_pdl(topk_slice_kernel<true>, dim3(1, M), dim3(kPartThreads), 0, stream, p);
     }
     p.cand_out = reinterpret_cast<uint2*>(workspace);
     p.list_out = nullptr;                       // the slices feed stage 2
-    topk_slice_kernel<false><<<dim3(G, M), kPartThreads, 0, stream>>>(p);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(topk_slice_kernel<false>, dim3(G, M), dim3(kPartThreads), 0, stream, p);
     if (e != cudaSuccess) return e;
     TopkParams q = p;
     q.logits = nullptr;
@@ -264,7 +307,7 @@ cudaError_t launch_topk(const void* logits, int dtype, uint32_t M, uint32_t N, s
     q.list_stride = p.k;
     q.row_stride = (size_t)G * p.k;
     q.list_out = reinterpret_cast<uint2*>(list_out);
-    return launch_merge(q, M, G, stream);
+    return launch_merge(q, M, stream);
 }
 
 cudaError_t launch_topk_sample(const void* logits, int dtype, uint32_t M, uint32_t N, uint32_t K, float temperature,
@@ -289,7 +332,7 @@ cudaError_t launch_topk_merge_sample(const void* pairs, uint32_t groups, size_t 
     q.temperature = temperature;
     q.u = u;
     q.out = out;
-    return launch_merge(q, M, groups, stream);
+    return launch_merge(q, M, stream);
 }
 
 }  // namespace vaicu
