@@ -7,6 +7,7 @@ Scope: what a graph of Linear nodes needs.  A net records once per input-shape
 set (prepare() + buffer binding + run(), vAi vai/engine/neural-net.cpp:406-518)
 and afterwards replays the recording (neural-net.h:391-438) — here a CUDA graph.
 """
+import collections
 import ctypes
 import enum
 import threading
@@ -262,6 +263,72 @@ class HostMappedBuffer:
         pass
 
 
+class _LoanedArray:
+    """Page-locked host memory that a caller holds as a numpy array: the array's base, so that the memory goes back to
+    its pool when the last view of it does."""
+
+    def __init__(self, pool, ptr):
+        self._pool, self._ptr = pool, ptr
+        self.__array_interface__ = {"data": (ptr, False), "shape": pool.shape, "typestr": pool.np_dtype.str, "version": 3}
+
+    def __del__(self):
+        self._pool.give_back(self._ptr)
+
+
+class _LoanPool:
+    """The page-locked arrays that one output of a recording is copied into and handed out in.  A large output (a
+    prefill's hidden state, one row of logits) reaches the caller in one copy that way; a staging buffer and a fresh
+    array cost a second pass over it and a page fault per 4 KB (513 KB of logits: 50 us of a 525 us step).  Two arrays are
+    made with the recording (a caller usually holds the last result while it asks for the next), at most LIMIT
+    exist; a caller that keeps more gets plain copies.  deque's append and pop are atomic, so arrays may die on any
+    thread, after the recording too."""
+    FIRST, LIMIT = 2, 4
+
+    def __init__(self, lib, nbytes, np_dtype, shape):
+        self.lib, self.nbytes, self.np_dtype, self.shape = lib, nbytes, np.dtype(np_dtype), tuple(shape)
+        self.spare = collections.deque()
+        self.made = 0
+        self.closed = False
+        while self.made < self.FIRST and self._make():
+            pass
+
+    def _make(self):
+        p = ctypes.c_void_p()
+        if self.lib.vaicu_host_alloc_pinned(self.nbytes, ctypes.byref(p)) != 0:
+            self.made = self.LIMIT          # no more to be had: copies from here on
+            return False
+        self.made += 1
+        self.spare.append(p.value)
+        return True
+
+    def take(self):
+        """A pointer to write to, or None when all are out."""
+        try:
+            return self.spare.pop()
+        except IndexError:
+            if self.made >= self.LIMIT or not self._make():
+                return None
+        return self.spare.pop()
+
+    def array(self, ptr):
+        return np.asarray(_LoanedArray(self, ptr))
+
+    def give_back(self, ptr):
+        self.spare.append(ptr)
+        if self.closed:
+            self.close()
+
+    def close(self):
+        """Frees what is spare; arrays still out free theirs when they die."""
+        self.closed = True
+        while True:
+            try:
+                ptr = self.spare.pop()
+            except IndexError:
+                return
+            self.lib.vaicu_host_free_pinned(ctypes.c_void_p(ptr))
+
+
 class Tensor:
     """Shape + dtype + host array and/or device buffer (vAi vai/engine/tensor.h:111-332).
     Copies share storage, as the reference's handle does."""
@@ -337,6 +404,10 @@ class Tensor:
             return np.array(raw).view(np.float16)
         return bits_to_f32(raw, Dtype.BF16)
 
+
+# Outputs handed out in page-locked arrays.  Below, the copy they save costs less than a command of its own; above, they
+# would pin too much of the host's memory.
+LOAN_MIN_BYTES, LOAN_MAX_BYTES = 64 << 10, 64 << 20
 
 # ---- graph: slots, nodes, flows ----------------------------------------------------
 
@@ -480,6 +551,7 @@ class _Recording:
         self.graph = None
         self.keep = []
         self.pinned = []        # page-locked host allocations made for this recording
+        self.loans = {}         # output -> the page-locked arrays it is handed out in
 
 
 class NeuralNet:
@@ -759,13 +831,15 @@ class NeuralNet:
             rec.graph = g
         # page-locked staging for the net's inputs and outputs, and a second recording that
         # brackets the same launches with the host<->device copies: one submission per call
-        rec.stage_in, rec.stage_out = {}, {}
+        rec.stage_in, rec.stage_out, rec.loans = {}, {}, {}
         for name, t in rec.input_tensors.items():
             rec.stage_in[name] = self._pinned(t.nbytes(), np.float32 if t.dtype == Dtype.F32 else np.uint16, t.shape)
         for name, t in rec.outputs.items():
             np_dtype = np.float32 if t.dtype == Dtype.F32 else np.uint16
             if isinstance(t.buffer, HostMappedBuffer):
                 rec.stage_out[name] = (t.buffer.view[:t.nbytes()].view(np_dtype).reshape(t.shape), None)
+            elif LOAN_MIN_BYTES <= t.nbytes() <= LOAN_MAX_BYTES:
+                rec.loans[name] = _LoanPool(lib, t.nbytes(), np_dtype, t.shape)
             else:
                 rec.stage_out[name] = self._pinned(t.nbytes(), np_dtype, t.shape)
         rec.graph_io = None
@@ -792,9 +866,21 @@ class NeuralNet:
     def _copies_out(self, rec):
         lib = self.device.lib
         for name, t in rec.outputs.items():
+            if name in rec.loans:       # a new destination on every call: _copy_loans
+                continue
             view, hp = rec.stage_out[name]
             if hp is not None:          # else the kernel wrote the host memory itself
                 _lib.check(lib.vaicu_memcpy_d2h(hp, t.ptr, view.nbytes, self.stream), "vaicu_memcpy_d2h")
+
+    def _copy_loans(self, rec):
+        """Enqueues the copies of the large outputs; {name: host array}, valid once the stream has been waited for."""
+        arrays = {}
+        for name, pool in rec.loans.items():
+            ptr = pool.take()
+            arrays[name] = pool.array(ptr) if ptr is not None else np.empty(pool.shape, dtype=pool.np_dtype)
+            _lib.check(self.device.lib.vaicu_memcpy_d2h(arrays[name].ctypes.data, rec.outputs[name].ptr, pool.nbytes, self.stream),
+                       "vaicu_memcpy_d2h")
+        return arrays
 
     def _play(self, ops):
         lib = self.device.lib
@@ -846,7 +932,7 @@ class NeuralNet:
             rec = self._record(fed)
             rec.calls = 0
             rec.h2d_bytes = sum(v.nbytes for v, _ in rec.stage_in.values())
-            rec.d2h_bytes = sum(v.nbytes for v, _ in rec.stage_out.values())
+            rec.d2h_bytes = sum(v.nbytes for v, _ in rec.stage_out.values()) + sum(pool.nbytes for pool in rec.loans.values())
             self._recordings[key] = rec
         for name, t in fed.items():
             np.copyto(rec.stage_in[name][0], t.host.reshape(rec.stage_in[name][0].shape))
@@ -856,6 +942,7 @@ class NeuralNet:
             self._copies_in(rec)
             self._play(rec.ops)
             self._copies_out(rec)
+        loaned = self._copy_loans(rec) if rec.loans else {}
         _lib.check(lib.vaicu_stream_sync(self.stream), "vaicu_stream_sync")
         # the kernels' bounded waits report through a device word: read it on the first
         # replay of a recording and then now and again, not on every step
@@ -866,7 +953,7 @@ class NeuralNet:
         outs = {}
         for name, t in rec.outputs.items():
             host = Tensor(t.shape, t.dtype)
-            host.host = rec.stage_out[name][0].copy()
+            host.host = loaned[name] if name in loaned else rec.stage_out[name][0].copy()
             outs[name] = host
         return outs[next(iter(outs))] if len(outs) == 1 else outs
 
@@ -883,6 +970,8 @@ class NeuralNet:
                 if g is not None:
                     lib.vaicu_graph_destroy(g)
             rec.graph = rec.graph_io = None
+            for pool in rec.loans.values():
+                pool.close()
             for p in rec.pinned:
                 lib.vaicu_host_free_pinned(p)
             rec.pinned = []
