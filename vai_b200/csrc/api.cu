@@ -1136,13 +1136,13 @@ int run_impl(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const 
         t.rs_rows = spec->rs_rows;
         t.rs_slot = spec->rs_slot;
         if (t.pair && spec->n_dst > 1u) {
-            // stores to peers go out as whole 128-byte row segments: one ring stage less, 16 KB of staging
+            // stores to peers go out as whole 128-byte row segments: one ring stage less, 32 KB of staging
             const uint32_t stage_bytes = 128u * 128u + (t.bn / 2u) * 128u;
-            const uint32_t staged_stages = (uint32_t)((kTcMaxSmem - 2048u - 16384u - 128u) / stage_bytes);
+            const uint32_t staged_stages = (uint32_t)((kTcMaxSmem - 2048u - kTcStagingBytes - 128u) / stage_bytes);
             if (staged_stages >= 3u) {
                 t.staged = 1u;
                 t.stages = staged_stages < t.stages ? staged_stages : t.stages;
-                smem = (size_t)t.stages * stage_bytes + 1024u + 256u + 16384u + 128u;
+                smem = (size_t)t.stages * stage_bytes + 1024u + 256u + kTcStagingBytes + 128u;
             }
         }
     }

@@ -7,13 +7,13 @@
 // (vai/shaders/linear-reduce.comp) fused into the store, and optionally the
 // GatedMul that follows a gate|value Linear (vai/nodes/gated-mul.h:9-20).
 //
-// Structure (one persistent CTA per SM, 192 threads):
-//   warp 0    one lane issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle)
+// Structure (one persistent CTA per SM, 384 threads):
+//   warps 0, 10, 11  one lane of each, k-block by k-block in turn, issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle)
 //             into a ring of shared-memory stages, signalled through mbarriers;
 //   warp 1    allocates tensor memory; one lane issues tcgen05.mma
 //             (cta_group::1, M = 128, N = bn, K = 16) and commits each stage back
 //             to the producer and each finished tile to the epilogue;
-//   warps 2-5 read the accumulator with tcgen05.ld (each warp owns 32 TMEM
+//   warps 2-9 read the accumulator with tcgen05.ld (a pair of warps owns 32 TMEM
 //             lanes), apply the epilogue and store.  Two accumulator buffers let
 //             the epilogue of tile i overlap the main loop of tile i+1.
 // "rows" operand A sits on the UMMA M axis (128 TMEM lanes), "cols" operand B on
@@ -35,8 +35,12 @@ namespace {
 constexpr uint32_t BLOCK_K = 64;          // 64 x 2 bytes = one 128-byte swizzle row
 constexpr uint32_t UMMA_K = 16;
 constexpr uint32_t TILE_ROWS = 128;       // UMMA M
-constexpr uint32_t kTcThreads = 192;        // producer warp, MMA warp, 4 epilogue warps
-constexpr uint32_t kTcThreadsSwap = 320;    // swapped kernel: 8 epilogue warps, two per quarter of the TMEM lanes
+// Warps: 0 producer, 1 MMA issuer, 2-9 epilogue (two per quarter of the TMEM lanes), 10-11 producers.  One thread takes
+// 600-800 cycles to wait for a stage, announce its bytes and issue its two or three copies (170 + 35 + 200 each,
+// measured), longer than the MMAs of most tiles and than HBM needs for a stage, so the k-blocks go round three producers.
+constexpr uint32_t kProducers = 3;
+constexpr uint32_t kEpiWarps = 8;
+constexpr uint32_t kTcThreads = 32u * (1u + kEpiWarps + kProducers);
 constexpr uint32_t kSpinLimit = 1u << 24; // bounded waits (each probe may sleep in hardware)
 
 // ---- PTX wrappers ---------------------------------------------------------
@@ -74,6 +78,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
     *abort_flag = 1u;
     return false;
+}
+
+// Whether the phase is over, without waiting: asked one k-block ahead, so that the answer is there when it is needed.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n"
+        " mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int32_t x, int32_t y)
@@ -311,6 +327,7 @@ __device__ __forceinline__ void finish_row16(const TcParams& p, float* v, float*
             for (int c = 0; c < 16; ++c) u[c] += t[c];
         }
     } else if (p.bias_mode != OPERAND_NONE) {   // [M,N] or repeating tables (never with GATE)
+#pragma unroll
         for (uint32_t c = 0; c < 16u; ++c) {
             const size_t i = (size_t)m * p.N + j0 + (c < n_valid ? c : n_valid - 1u);
             v[c] += load_as_f32(p.bias, p.b_dtype, p.bias_mode == OPERAND_MODULO ? i % p.bias_elems : i);
@@ -319,8 +336,10 @@ __device__ __forceinline__ void finish_row16(const TcParams& p, float* v, float*
     if (p.res_mode == OPERAND_FULL && pre && pre->valid) res_unpack(p.o_dtype, *pre, t);
     else if (p.res_mode == OPERAND_FULL) load16(p.res, p.o_dtype, flat0, n_valid, t);
     else if (p.res_mode == OPERAND_PER_COLUMN) load16(p.res, p.o_dtype, j0, n_valid, t);
-    else if (p.res_mode == OPERAND_MODULO)
+    else if (p.res_mode == OPERAND_MODULO) {
+#pragma unroll
         for (uint32_t c = 0; c < 16u; ++c) t[c] = load_as_f32(p.res, p.o_dtype, (flat0 + (c < n_valid ? c : n_valid - 1u)) % p.res_elems);
+    }
     const bool before = p.res_mode != OPERAND_NONE && p.residual_order == VAICU_RESIDUAL_BEFORE_EPILOGUE;
     const bool after = p.res_mode != OPERAND_NONE && !before;
     if (before) {
@@ -353,6 +372,7 @@ __device__ __forceinline__ void finish_col16(const TcParams& p, float* v, float*
 #pragma unroll
         for (int c = 0; c < 16; ++c) { v[c] += bias_n; if (GATE) u[c] += bias_up; }
     } else if (p.bias_mode != OPERAND_NONE) {
+#pragma unroll
         for (uint32_t c = 0; c < 16u; ++c) {
             const uint32_t m = m0 + c < p.M ? m0 + c : p.M - 1u;
             const size_t i = (size_t)m * p.N + n;
@@ -371,6 +391,7 @@ __device__ __forceinline__ void finish_col16(const TcParams& p, float* v, float*
 #pragma unroll
         for (uint32_t c = 0; c < 16u; ++c) t[c] = r;
     } else if (p.res_mode != OPERAND_NONE) {
+#pragma unroll
         for (uint32_t c = 0; c < 16u; ++c) {
             const uint32_t m = m0 + c < p.M ? m0 + c : p.M - 1u;
             t[c] = load_as_f32(p.res, p.o_dtype, ((size_t)m * out_cols + n) % p.res_elems);
@@ -417,7 +438,9 @@ __device__ __forceinline__ void emit_rows16(const TcParams& p, float* v, float* 
         const size_t at = (size_t)m * width + (j0 - first);
         if (n_valid == 16u && ((at * osz) % 16u == 0u)) store16(p.dst[j], p.o_dtype, at, v, true);
         else
-            for (uint32_t c = 0; c < n_valid; ++c) store_from_f32(p.dst[j], p.o_dtype, at + c, v[c]);
+#pragma unroll
+            for (uint32_t c = 0; c < 16u; ++c)
+                if (c < n_valid) store_from_f32(p.dst[j], p.o_dtype, at + c, v[c]);
         return;
     }
     uint32_t owner;
@@ -430,7 +453,9 @@ __device__ __forceinline__ void emit_rows16(const TcParams& p, float* v, float* 
         void* dst = p.n_dst == 1u ? p.O : p.dst[d];
         if (vec_ok) store16(dst, p.o_dtype, flat0, v, true);
         else
-            for (uint32_t c = 0; c < n_valid; ++c) store_from_f32(dst, p.o_dtype, flat0 + c, v[c]);
+#pragma unroll
+            for (uint32_t c = 0; c < 16u; ++c)
+                if (c < n_valid) store_from_f32(dst, p.o_dtype, flat0 + c, v[c]);
     }
 }
 
@@ -442,6 +467,7 @@ __device__ __forceinline__ void emit_cols16(const TcParams& p, float* v, float* 
 {
     finish_col16<GATE>(p, v, u, n, m0, out_cols, bias_n, bias_up);
     if (p.rs_rows) {                       // row-parallel run: each activation row goes to its owner's staging
+#pragma unroll
         for (uint32_t c = 0; c < 16u; ++c) {
             if (m0 + c >= p.M) break;
             uint32_t owner;
@@ -560,7 +586,7 @@ __device__ __forceinline__ void tc_trace(uint32_t slot)
 //       bn/2 value rows; swap: the A stage holds 128 gate rows then 128 value rows
 //       and two MMAs per k-step fill two accumulators.
 template <bool SWAP, bool GATE>
-__global__ void __launch_bounds__(SWAP ? kTcThreadsSwap : kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ CUtensorMap tmap_a1, const __grid_constant__ CUtensorMap tmap_a2, const TcParams p)
 {
@@ -606,11 +632,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        // epilogue warps: 4, or 8 that share each quarter of the accumulator's lanes by column chunks (swapped
-        // kernel: its CTAs often hold a single tile, whose epilogue nothing overlaps)
-        const uint32_t epi_warps = (blockDim.x >> 5) - 2u;
-        for (uint32_t b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], epi_warps); }
-        mbar_init(fold_in, epi_warps);
+        // 8 epilogue warps: a CTA that holds a single tile has nothing to hide its epilogue behind
+        for (uint32_t b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], kEpiWarps); }
+        mbar_init(fold_in, kEpiWarps);
         mbar_init(fold_out, 1);
         *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -637,10 +661,11 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // The launch after this one may begin its prologue now (it waits before it touches our results).
     launch_dependents();
 
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
+    if (warp == 0 || warp >= 2u + kEpiWarps) {
+        // ---------------- TMA producers, k-block by k-block in turn ----------------
         if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
+            const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps;
+            uint32_t stage = 0, phase = 0, turn = 0;
             bool ok = true;
             // One k-block of one operand into its stage.  "A" sits on the UMMA M axis, "B" on N.
             auto load_a = [&](uint32_t st, uint32_t kb, uint32_t ta) {
@@ -684,25 +709,29 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     // follow once it has completed.  (Weights are operand A when swapped, else B.)
                     first = false;
                     const uint32_t npre = (kb1 - kb0 < stages) ? kb1 - kb0 : stages;
-                    for (uint32_t i = 0; i < npre; ++i) {        // the ring is empty: no wait needed
+                    for (uint32_t i = me; i < npre; i += kProducers) {        // the ring is empty: no wait needed
                         mbar_expect_tx(&full_bar[i], tx_bytes);
                         if (SWAP) load_a(i, kb0 + i, ta); else load_b(i, kb0 + i, tb);
                     }
                     TC_TRACE(2);
                     dependency_wait();
                     TC_TRACE(3);
-                    for (uint32_t i = 0; i < npre; ++i) {
+                    for (uint32_t i = me; i < npre; i += kProducers) {
                         if (SWAP) load_b(i, kb0 + i, tb); else load_a(i, kb0 + i, ta);
                     }
                     kb = kb0 + npre;
+                    turn = npre % kProducers;
                     stage = npre == stages ? 0u : npre;
                     phase = npre == stages ? 1u : 0u;
                 }
                 for (; kb < kb1; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-                    mbar_expect_tx(&full_bar[stage], tx_bytes);
-                    load_a(stage, kb, ta);
-                    load_b(stage, kb, tb);
+                    if (turn == me) {
+                        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx(&full_bar[stage], tx_bytes);
+                        load_a(stage, kb, ta);
+                        load_b(stage, kb, tb);
+                    }
+                    if (++turn == kProducers) turn = 0;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -713,7 +742,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
             uint32_t stage = 0, phase = 0, iter = 0;
-            bool ok = true;
+            bool ok = true, ready = false;           // ready: the stage at hand was seen full a k-block ago
             for (uint32_t w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++iter) {
                 const uint32_t tile = w / p.splits, z = w - tile * p.splits;
                 const uint32_t kb0 = z * p.kb_per_split;
@@ -723,7 +752,9 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * acc_cols;
                 for (uint32_t kb = kb0; kb < kb1; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+                    if (!ready && !mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+                    const uint32_t next = stage + 1u == stages ? 0u : stage + 1u;
+                    ready = mbar_test(&full_bar[next], next ? phase : phase ^ 1u);
                     tc_fence_after();
                     if (iter == 0 && kb == kb0) TC_TRACE(5);
                     const uint32_t sa = smem_u32(smem + (size_t)stage * stage_bytes);
@@ -751,7 +782,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // ---------------- epilogue warps ----------------
         const uint32_t q = warp & 3u;                    // TMEM lane quarter this warp may read
         const uint32_t row_in_tile = q * 32u + lane;
-        const uint32_t col_groups = ((blockDim.x >> 5) - 2u) >> 2;   // warps per lane quarter: 1 or 2
+        constexpr uint32_t col_groups = kEpiWarps / 4u;              // warps per lane quarter
         const uint32_t col_group = (warp - 2u) >> 2;                 // this warp's share of the 16-column chunks
         const uint32_t out_cols = GATE ? p.H : p.N;      // width of O
         const uint32_t osz = p.partial ? 4u : dtype_size(p.o_dtype);
@@ -915,9 +946,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if (threadIdx.x == 64u) TC_TRACE(10);
         cluster_sync_all();
         if (threadIdx.x == 64u) TC_TRACE(11);
-        if (warp >= 2 && !*abort_flag) {
+        if (warp >= 2u && warp < 2u + kEpiWarps && !*abort_flag) {
             const uint32_t q = warp & 3u, row_in_tile = q * 32u + lane;
-            const uint32_t col_groups = ((blockDim.x >> 5) - 2u) >> 2, col_group = (warp - 2u) >> 2;
+            constexpr uint32_t col_groups = kEpiWarps / 4u;
+            const uint32_t col_group = (warp - 2u) >> 2;
             const uint32_t tile = blockIdx.x / p.splits, z = blockIdx.x - tile * p.splits;
             uint32_t ta, tb;
             tile_coords(p, tile, ta, tb);
@@ -1065,12 +1097,12 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     uint64_t* acc_empty = acc_full + 2;           // [2], used in the leader
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    // 4 KB per epilogue warp for the staged stores (present when p.staged)
+    // 4 KB per epilogue warp for the staged stores (kTcStagingBytes, present when p.staged)
     uint8_t* staging = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tmem_slot + 2) + 127u) & ~(uintptr_t)127u);
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-        for (uint32_t b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }   // 4 warps x 2 CTAs
+        for (uint32_t b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 2u * kEpiWarps); }   // both CTAs' epilogues
         *abort_flag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1094,10 +1126,11 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // The launch after this one may begin its prologue now (it waits before it touches our results).
     launch_dependents();
 
-    if (warp == 0) {
-        // ---------------- TMA producer (both CTAs) ----------------
+    if (warp == 0 || warp >= 2u + kEpiWarps) {
+        // ---------------- TMA producers (both CTAs), k-block by k-block in turn ----------------
         if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
+            const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps;
+            uint32_t stage = 0, phase = 0, turn = 0;
             bool ok = true;
             bool first = true;
             for (uint32_t w = cluster_id; w < num_work && ok; w += num_clusters) {
@@ -1126,33 +1159,37 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     // follow once it has completed.
                     first = false;
                     const uint32_t npre = (kb1 - kb0 < stages) ? kb1 - kb0 : stages;
-                    for (uint32_t i = 0; i < npre; ++i) {        // the ring is empty: no wait needed
+                    for (uint32_t i = me; i < npre; i += kProducers) {        // the ring is empty: no wait needed
                         if (rank == 0u) mbar_expect_tx(&full_bar[i], 2u * item_bytes);
                         tma_load_2d_pair(smem + (size_t)i * stage_bytes + a_bytes, mb, map_to_cta(smem_u32(&full_bar[i]), 0u),
                                          (int32_t)((kb0 + i) * BLOCK_K), yb);
                     }
                     dependency_wait();
-                    for (uint32_t i = 0; i < npre; ++i)
+                    for (uint32_t i = me; i < npre; i += kProducers)
                         tma_load_2d_pair(smem + (size_t)i * stage_bytes, &tmap_a, map_to_cta(smem_u32(&full_bar[i]), 0u),
                                          (int32_t)((kb0 + i) * BLOCK_K), ya);
                     kb = kb0 + npre;
                     stage = npre == stages ? 0u : npre;
                     phase = npre == stages ? 1u : 0u;
+                    turn = npre % kProducers;
                 }
                 for (; kb < kb1; ++kb) {
-                    if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-                    uint8_t* sa = smem + (size_t)stage * stage_bytes;
-                    if (rank == 0u) mbar_expect_tx(&full_bar[stage], 2u * item_bytes);   // both CTAs' boxes
-                    const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0u);
-                    const int32_t kx = (int32_t)(kb * BLOCK_K);
-                    tma_load_2d_pair(sa, &tmap_a, bar, kx, ya);
-                    tma_load_2d_pair(sa + a_bytes, mb, bar, kx, yb);
+                    if (turn == me) {
+                        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+                        uint8_t* sa = smem + (size_t)stage * stage_bytes;
+                        if (rank == 0u) mbar_expect_tx(&full_bar[stage], 2u * item_bytes);   // both CTAs' boxes
+                        const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0u);
+                        const int32_t kx = (int32_t)(kb * BLOCK_K);
+                        tma_load_2d_pair(sa, &tmap_a, bar, kx, ya);
+                        tma_load_2d_pair(sa + a_bytes, mb, bar, kx, yb);
+                    }
+                    if (++turn == kProducers) turn = 0;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
             }
             if (first) dependency_wait();
             // the leader's last commits land on this CTA's barriers before it may leave
-            for (uint32_t s = 0; s < stages && ok; ++s) {
+            for (uint32_t s = 0; s < stages && ok && me == 0u; ++s) {
                 if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) ok = false;
                 if (++stage == stages) { stage = 0; phase ^= 1u; }
             }
@@ -1161,7 +1198,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // ---------------- MMA issuer (leader CTA only) ----------------
         if (lane == 0 && rank == 0u) {
             uint32_t stage = 0, phase = 0, iter = 0;
-            bool ok = true;
+            bool ok = true, ready = false;           // ready: the stage at hand was seen full a k-block ago
             for (uint32_t w = cluster_id; w < num_work && ok; w += num_clusters, ++iter) {
                 uint32_t tile, z, strip, bw;
                 work_item(p, w, tile, z, strip, bw);
@@ -1173,7 +1210,9 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * acc_cols;
                 for (uint32_t kb = kb0; kb < kb1; ++kb) {
-                    if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+                    if (!ready && !mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+                    const uint32_t next = stage + 1u == stages ? 0u : stage + 1u;
+                    ready = mbar_test(&full_bar[next], next ? phase : phase ^ 1u);
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + (size_t)stage * stage_bytes);
                     const uint64_t a_desc = make_smem_desc(sa);
@@ -1212,7 +1251,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (res_rows) {
                 const uint32_t rsz = dtype_size(p.o_dtype);
                 const uint8_t* rp = reinterpret_cast<const uint8_t*>(p.res) + ((size_t)m * out_cols + j_item) * rsz;
-                const uint32_t span = (j_item + ncols <= out_cols ? ncols : (j_item < out_cols ? out_cols - j_item : 0u)) * rsz;
+                const uint32_t span = (warp >= 6u ? 0u : j_item + ncols <= out_cols ? ncols : (j_item < out_cols ? out_cols - j_item : 0u)) * rsz;
                 for (uint32_t b = 0; b < span; b += 128u) asm volatile("prefetch.global.L2 [%0];" ::"l"(rp + b));
             }
             const uint32_t buf = iter & 1u, use = iter >> 1;
@@ -1221,15 +1260,17 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const uint32_t t_row = tmem_base + ((q * 32u) << 16) + buf * acc_cols;
             // columns per 128-byte row segment of the output
             const uint32_t seg_cols = 128u / osz;
+            // the two warps of a lane quarter take half of the item's 16-column chunks each
+            const uint32_t c_mid = ncols / 32u * 16u, c_begin = warp < 6u ? 0u : c_mid, c_end = warp < 6u ? c_mid : ncols;
             ResRaw res_next;
-            res_issue(p, m, j_item, out_cols, res_next);
-            for (uint32_t c0 = 0; c0 < ncols;) {
+            res_issue(p, m, j_item + c_begin, out_cols, res_next);
+            for (uint32_t c0 = c_begin; c0 < c_end;) {
                 const uint32_t j_seg = j_item + c0;
-                const bool stage_it = p.staged && !p.partial && c0 + seg_cols <= ncols && j_seg + seg_cols <= out_cols &&
+                const bool stage_it = p.staged && !p.partial && c0 + seg_cols <= c_end && j_seg + seg_cols <= out_cols &&
                                       p.o_aligned16 && (((size_t)p.ldo * osz) % 16u == 0u) && (((size_t)(p.col0 + j_seg) * osz) % 16u == 0u);
                 if (!stage_it) {
                     const ResRaw res_cur = res_next;
-                    if (c0 + 16u < ncols) res_issue(p, m, j_seg + 16u, out_cols, res_next);      // in flight while this chunk is finished
+                    if (c0 + 16u < c_end) res_issue(p, m, j_seg + 16u, out_cols, res_next);      // in flight while this chunk is finished
                     uint32_t r0[16], r1[16];
                     tmem_ld16(t_row + c0, r0);
                     if (GATE) tmem_ld16(t_row + c0 + bh, r1);
@@ -1240,7 +1281,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
                 // 1. this thread's row: seg_cols finished values -> its 128-byte line of the warp's staging
                 //    block, 16-byte chunks XOR-swizzled by the row so that the 32 lanes hit distinct banks
-                uint8_t* mine = staging + (size_t)q * 4096u + (size_t)lane * 128u;
+                uint8_t* mine = staging + (size_t)(warp - 2u) * 4096u + (size_t)lane * 128u;
                 for (uint32_t g = 0; g < seg_cols; g += 16u) {
                     uint32_t r0[16], r1[16];
                     tmem_ld16(t_row + c0 + g, r0);
@@ -1282,7 +1323,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
                 for (uint32_t it = 0; it < 8u; ++it) {
                     const uint32_t rr = it * 4u + (lane >> 3), chunk = lane & 7u;
-                    const uint4 val = *reinterpret_cast<const uint4*>(staging + (size_t)q * 4096u + (size_t)rr * 128u + ((chunk ^ (rr & 7u)) * 16u));
+                    const uint4 val = *reinterpret_cast<const uint4*>(staging + (size_t)(warp - 2u) * 4096u + (size_t)rr * 128u + ((chunk ^ (rr & 7u)) * 16u));
                     if (m_base + rr < p.M) {
                         uint32_t owner;
                         size_t row;
@@ -1379,8 +1420,8 @@ static cudaError_t launch_variant(const CUtensorMap& ma, const CUtensorMap& mb, 
     static SmemOptIn optin;
     if (cudaError_t e = optin.ensure(kern, (int)kTcMaxSmem); e != cudaSuccess) return e;
     if (SWAP && !GATE && p.cfold)
-        return launch_pdl_cluster(kern, dim3((unsigned)grid), dim3(kTcThreadsSwap), smem, stream, p.cfold, ma, mb, ma1, ma2, p);
-    return launch_pdl(kern, dim3((unsigned)grid), dim3(SWAP ? kTcThreadsSwap : kTcThreads), smem, stream, ma, mb, ma1, ma2, p);
+        return launch_pdl_cluster(kern, dim3((unsigned)grid), dim3(kTcThreads), smem, stream, p.cfold, ma, mb, ma1, ma2, p);
+    return launch_pdl(kern, dim3((unsigned)grid), dim3(kTcThreads), smem, stream, ma, mb, ma1, ma2, p);
 }
 
 // Clusters of `cluster` CTAs of the swapped kernel that can be resident at once.
@@ -1396,7 +1437,7 @@ cudaError_t tc_swap_max_clusters(size_t smem, unsigned cluster, int* clusters)
     attr[0].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cluster, 1, 1);
-    cfg.blockDim = dim3(kTcThreadsSwap, 1, 1);
+    cfg.blockDim = dim3(kTcThreads, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;

@@ -8,6 +8,7 @@
 namespace vaicu {
 
 constexpr size_t kTcMaxSmem = 227u * 1024u;   // opt-in shared memory per CTA on sm_100
+constexpr uint32_t kTcStagingBytes = 8u * 4096u;   // CTA-pair kernel, several destinations: 4 KB per epilogue warp
 
 // How bias / residual are indexed, resolved on the host so the epilogue avoids a
 // 64-bit modulo per element (rule: vAi vai/nodes/linear.h:2333-2338).
