@@ -92,6 +92,20 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity)
     return ok != 0;
 }
 
+// The producing and issuing roles run with all 32 lanes and let one of them act: copies and MMAs take their operands
+// from uniform registers, which the compiler only fills directly where the whole warp goes the same way (with the role
+// confined to one lane an MMA cost 69 cycles to issue, four per k-block).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(e));
+    return e != 0;
+}
+__device__ __forceinline__ bool warp_mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag)
+{
+    return __all_sync(0xFFFFFFFFu, mbar_wait(bar, parity, abort_flag));
+}
+
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int32_t x, int32_t y)
 {
     asm volatile(
@@ -594,7 +608,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // 1024-byte alignment is required by the 128-byte swizzle atoms
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const uint32_t bn = p.bn;
     if (threadIdx.x == 0) TC_TRACE(0);
     // wide: two 128-row A boxes per stage and two MMAs per k-step give a 256-row tile;
@@ -663,7 +677,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     if (warp == 0 || warp >= 2u + kEpiWarps) {
         // ---------------- TMA producers, k-block by k-block in turn ----------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps;
             uint32_t stage = 0, phase = 0, turn = 0;
             bool ok = true;
@@ -710,6 +725,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     first = false;
                     const uint32_t npre = (kb1 - kb0 < stages) ? kb1 - kb0 : stages;
                     for (uint32_t i = me; i < npre; i += kProducers) {        // the ring is empty: no wait needed
+                        if (!leader) continue;
                         mbar_expect_tx(&full_bar[i], tx_bytes);
                         if (SWAP) load_a(i, kb0 + i, ta); else load_b(i, kb0 + i, tb);
                     }
@@ -717,6 +733,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     dependency_wait();
                     TC_TRACE(3);
                     for (uint32_t i = me; i < npre; i += kProducers) {
+                        if (!leader) continue;
                         if (SWAP) load_b(i, kb0 + i, tb); else load_a(i, kb0 + i, ta);
                     }
                     kb = kb0 + npre;
@@ -726,10 +743,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 }
                 for (; kb < kb1; ++kb) {
                     if (turn == me) {
-                        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-                        mbar_expect_tx(&full_bar[stage], tx_bytes);
-                        load_a(stage, kb, ta);
-                        load_b(stage, kb, tb);
+                        if (!warp_mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+                        if (leader) {
+                            mbar_expect_tx(&full_bar[stage], tx_bytes);
+                            load_a(stage, kb, ta);
+                            load_b(stage, kb, tb);
+                        }
                     }
                     if (++turn == kProducers) turn = 0;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -740,7 +759,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             uint32_t stage = 0, phase = 0, iter = 0;
             bool ok = true, ready = false;           // ready: the stage at hand was seen full a k-block ago
             for (uint32_t w = blockIdx.x; w < num_work && ok; w += gridDim.x, ++iter) {
@@ -748,19 +768,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                 const uint32_t kb0 = z * p.kb_per_split;
                 const uint32_t kb1 = (kb0 + p.kb_per_split < p.kblocks) ? kb0 + p.kb_per_split : p.kblocks;
                 const uint32_t buf = iter % acc_bufs, use = iter / acc_bufs;
-                if (!mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+                if (!warp_mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * acc_cols;
                 for (uint32_t kb = kb0; kb < kb1; ++kb) {
-                    if (!ready && !mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+                    if (!ready && !warp_mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
                     const uint32_t next = stage + 1u == stages ? 0u : stage + 1u;
-                    ready = mbar_test(&full_bar[next], next ? phase : phase ^ 1u);
+                    ready = __all_sync(0xFFFFFFFFu, mbar_test(&full_bar[next], next ? phase : phase ^ 1u));
                     tc_fence_after();
                     if (iter == 0 && kb == kb0) TC_TRACE(5);
                     const uint32_t sa = smem_u32(smem + (size_t)stage * stage_bytes);
                     const uint32_t sb = sa + a_bytes;
                     const uint64_t a_desc = make_smem_desc(sa);
                     const uint64_t b_desc = make_smem_desc(sb);
+                    if (leader) {
 #pragma unroll
                     for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k) {
                         const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
@@ -772,9 +793,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                         }
                     }
                     umma_commit(&empty_bar[stage]);     // stage reusable once these MMAs retire
+                    }
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
-                if (ok) umma_commit(&acc_full[buf]);     // accumulator complete
+                if (ok && leader) umma_commit(&acc_full[buf]);     // accumulator complete
                 TC_TRACE(6);
             }
         }
@@ -1081,7 +1103,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31u;
     const uint32_t rank = cluster_ctarank();
     const uint32_t cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
     const uint32_t bn = p.bn, half = bn / 2u;
@@ -1128,7 +1150,8 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
     if (warp == 0 || warp >= 2u + kEpiWarps) {
         // ---------------- TMA producers (both CTAs), k-block by k-block in turn ----------------
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps;
             uint32_t stage = 0, phase = 0, turn = 0;
             bool ok = true;
@@ -1160,13 +1183,14 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     first = false;
                     const uint32_t npre = (kb1 - kb0 < stages) ? kb1 - kb0 : stages;
                     for (uint32_t i = me; i < npre; i += kProducers) {        // the ring is empty: no wait needed
+                        if (!leader) continue;
                         if (rank == 0u) mbar_expect_tx(&full_bar[i], 2u * item_bytes);
                         tma_load_2d_pair(smem + (size_t)i * stage_bytes + a_bytes, mb, map_to_cta(smem_u32(&full_bar[i]), 0u),
                                          (int32_t)((kb0 + i) * BLOCK_K), yb);
                     }
                     dependency_wait();
                     for (uint32_t i = me; i < npre; i += kProducers)
-                        tma_load_2d_pair(smem + (size_t)i * stage_bytes, &tmap_a, map_to_cta(smem_u32(&full_bar[i]), 0u),
+                        if (leader) tma_load_2d_pair(smem + (size_t)i * stage_bytes, &tmap_a, map_to_cta(smem_u32(&full_bar[i]), 0u),
                                          (int32_t)((kb0 + i) * BLOCK_K), ya);
                     kb = kb0 + npre;
                     stage = npre == stages ? 0u : npre;
@@ -1175,13 +1199,15 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
                 for (; kb < kb1; ++kb) {
                     if (turn == me) {
-                        if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+                        if (!warp_mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
                         uint8_t* sa = smem + (size_t)stage * stage_bytes;
-                        if (rank == 0u) mbar_expect_tx(&full_bar[stage], 2u * item_bytes);   // both CTAs' boxes
                         const uint32_t bar = map_to_cta(smem_u32(&full_bar[stage]), 0u);
                         const int32_t kx = (int32_t)(kb * BLOCK_K);
-                        tma_load_2d_pair(sa, &tmap_a, bar, kx, ya);
-                        tma_load_2d_pair(sa + a_bytes, mb, bar, kx, yb);
+                        if (leader) {
+                            if (rank == 0u) mbar_expect_tx(&full_bar[stage], 2u * item_bytes);   // both CTAs' boxes
+                            tma_load_2d_pair(sa, &tmap_a, bar, kx, ya);
+                            tma_load_2d_pair(sa + a_bytes, mb, bar, kx, yb);
+                        }
                     }
                     if (++turn == kProducers) turn = 0;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
@@ -1190,13 +1216,14 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if (first) dependency_wait();
             // the leader's last commits land on this CTA's barriers before it may leave
             for (uint32_t s = 0; s < stages && ok && me == 0u; ++s) {
-                if (!mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) ok = false;
+                if (!warp_mbar_wait(&empty_bar[stage], phase ^ 1u, abort_flag)) ok = false;
                 if (++stage == stages) { stage = 0; phase ^= 1u; }
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (leader CTA only) ----------------
-        if (lane == 0 && rank == 0u) {
+        if (rank == 0u) {
+            const bool leader = elect_one();
             uint32_t stage = 0, phase = 0, iter = 0;
             bool ok = true, ready = false;           // ready: the stage at hand was seen full a k-block ago
             for (uint32_t w = cluster_id; w < num_work && ok; w += num_clusters, ++iter) {
@@ -1206,24 +1233,26 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 const uint32_t kb0 = z * p.kb_per_split;
                 const uint32_t kb1 = (kb0 + p.kb_per_split < p.kblocks) ? kb0 + p.kb_per_split : p.kblocks;
                 const uint32_t buf = iter & 1u, use = iter >> 1;
-                if (!mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+                if (!warp_mbar_wait(&acc_empty[buf], (use & 1u) ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * acc_cols;
                 for (uint32_t kb = kb0; kb < kb1; ++kb) {
-                    if (!ready && !mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+                    if (!ready && !warp_mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
                     const uint32_t next = stage + 1u == stages ? 0u : stage + 1u;
-                    ready = mbar_test(&full_bar[next], next ? phase : phase ^ 1u);
+                    ready = __all_sync(0xFFFFFFFFu, mbar_test(&full_bar[next], next ? phase : phase ^ 1u));
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + (size_t)stage * stage_bytes);
                     const uint64_t a_desc = make_smem_desc(sa);
                     const uint64_t b_desc = make_smem_desc(sa + a_bytes);
+                    if (leader) {
 #pragma unroll
-                    for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k)
-                        umma_f16_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-                    umma_commit_pair(&empty_bar[stage]);    // frees the stage in both CTAs
+                        for (uint32_t k = 0; k < BLOCK_K / UMMA_K; ++k)
+                            umma_f16_pair(d_tmem, a_desc + 2u * k, b_desc + 2u * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        umma_commit_pair(&empty_bar[stage]);    // frees the stage in both CTAs
+                    }
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
-                if (ok) umma_commit_pair(&acc_full[buf]);    // wakes the epilogues of both CTAs
+                if (ok && leader) umma_commit_pair(&acc_full[buf]);    // wakes the epilogues of both CTAs
             }
         }
     } else {
