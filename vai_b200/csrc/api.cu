@@ -242,6 +242,42 @@ bool tc_eligible(const vaicu_linear_desc& d)
     return true;
 }
 
+// Columns per tile and K splits of the CTA-pair kernel: the cheapest by a model of its time in microseconds,
+//   rounds of tiles x k-blocks per split x (time of a k-block) + (epilogue per column) x bn + (fold of the splits).
+// A k-block takes 0.19 us at 64 columns and hardly more up to 128 (issue and L2 set the pace), 0.255 at 192, 0.32 at 256
+// (the MMAs do); a last round of few tiles runs as column strips.  Measured over 19 layers x 160-2000 rows, all
+// five widths and up to 8 splits: the choice is 0.5 % off the best on average, 14 % at most (whole-wave rule before: 5 %).
+// From two full rounds of 256-column tiles on those are taken: wider tiles read the operands less often.
+uint32_t choose_pair_tile(const vaicu_linear_desc& d, uint32_t units, uint32_t* splits)
+{
+    const bool gate = d.gate_fuse != 0;
+    const uint32_t H = gate ? d.N / 2u : d.N, tiles_m = ceil_div(d.M, 256u), kblocks = ceil_div(d.K, 64u);
+    const uint32_t cand[5] = {64u, 96u, 128u, 192u, 256u};
+    const double per_kb[5] = {0.19, 0.225, 0.22, 0.255, 0.32};
+    *splits = 1u;
+    if (tiles_m * ceil_div(H, gate ? 128u : 256u) >= 2u * units) return 256u;
+    uint32_t best_bn = 256u;
+    double best = 1e30;
+    for (int i = 0; i < 5; ++i) {
+        const uint32_t bn = cand[i], tiles = tiles_m * ceil_div(H, gate ? bn / 2u : bn);
+        for (uint32_t s : {1u, 2u, 3u, 4u, 6u, 8u}) {
+            if (s > 1u && (kblocks / s < 4u || tiles * s > 2u * units || d.split_size)) continue;
+            const uint32_t kps = ceil_div(kblocks, s), real = ceil_div(kblocks, kps);
+            const uint32_t full = tiles * real / units, rem = tiles * real % units;
+            double cost = 0.015 * bn + full * kps * per_kb[i];
+            if (rem) {
+                uint32_t width = bn;
+                for (uint32_t c = 2u; real == 1u && full && c <= 4u; c *= 2u)
+                    if (bn % c == 0u && (bn / c) % 32u == 0u && rem * c <= units) width = bn / c;
+                cost += kps * (width == bn ? per_kb[i] : (width >= 128u ? per_kb[2] : (width >= 96u ? per_kb[1] : per_kb[0])));
+            }
+            if (real > 1u) cost += 2.5 + 0.35e-6 * (real + 1.0) * d.M * d.N * 4.0;
+            if (cost < best) { best = cost; best_bn = bn; *splits = real; }
+        }
+    }
+    return best_bn;
+}
+
 // Tile / split choice of the tensor-core kernel (the role selectLinearTile plays
 // in the reference, vAi linear.h:2101-2119): fill the SMs with whole waves of
 // the widest tile, and split K only when the tile grid cannot occupy them.
@@ -256,7 +292,7 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
     t.M = d.M; t.N = d.N; t.K = d.K; t.H = H;
     t.kblocks = ceil_div(d.K, 64u);
     t.grp_t1 = t.grp_t2 = kNoGroup;
-    uint32_t bn;
+    uint32_t bn, pair_splits = 1u;
     t.tile_rows = 128u;
     if (swap) {
         bn = (uint32_t)align_up(d.M, 16u);
@@ -272,7 +308,9 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
         const uint32_t boxes = gate ? 2u : 1u;
         uint32_t best_rows = 128u;
         uint64_t best_cost = ~0ull;
-        for (uint32_t rows = 128u; rows >= 32u && !d.split_size; rows -= 8u) {
+        // At least 64 rows without a gate: below, a layer of 2560-4700 rows would just fit the SMs unsplit with a quarter of
+        // the loads in flight (K = 8192, N = 3072 at 24 rows of activations: 38 us in 40-row tiles, 14 us split).
+        for (uint32_t rows = 128u; rows >= (gate ? 32u : 64u) && !d.split_size; rows -= 8u) {
             if (boxes * rows < bn) break;
             const uint32_t tiles = ceil_div(H, rows) * t.tiles_b;
             if (tiles * 2u <= sms) continue;
@@ -288,22 +326,23 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
         bool pair = d.M > 128u;
         if (pl->tune.tc_pair >= 0) pair = pl->tune.tc_pair != 0;
         // output columns per tile: bn (bn / 2 with gate)
-        const uint32_t cand[3] = {256u, 128u, 64u};
-        const uint32_t rows = pair ? 256u : 128u, units = pair ? sms / 2u : sms;
-        double best = -1.0;
         bn = 256u;
-        for (uint32_t c : cand) {
-            const uint32_t out_cols = gate ? c / 2u : c;
-            const uint32_t tiles = ceil_div(d.M, rows) * ceil_div(H, out_cols);
-            const uint32_t waves = ceil_div(tiles, units);
-            double eff = (double)tiles / ((double)waves * units);
-            // narrower tiles re-read the activations more often and issue shorter MMAs
-            // (measured on 8192 x 3072 x 3072: 1256 / 888 TFLOP/s for 256 / 128 on pairs)
-            if (pair) eff *= (c == 256u) ? 1.0 : (c == 128u ? 0.70 : 0.45);
-            else eff *= (c == 256u) ? 1.0 : (c == 128u ? 0.88 : 0.70);
-            // a tile wider than the whole output is wasted work
-            if (out_cols > (uint32_t)align_up(H, 16u) && c != 64u) eff *= (double)H / out_cols;
-            if (eff > best) { best = eff; bn = c; }
+        if (pair) {
+            bn = choose_pair_tile(d, sms / 2u, &pair_splits);
+        } else {
+            const uint32_t cand[3] = {256u, 128u, 64u};
+            double best = -1.0;
+            for (uint32_t c : cand) {
+                const uint32_t out_cols = gate ? c / 2u : c;
+                const uint32_t tiles = ceil_div(d.M, 128u) * ceil_div(H, out_cols);
+                const uint32_t waves = ceil_div(tiles, sms);
+                double eff = (double)tiles / ((double)waves * sms);
+                // narrower tiles re-read the activations more often and issue shorter MMAs
+                eff *= (c == 256u) ? 1.0 : (c == 128u ? 0.88 : 0.70);
+                // a tile wider than the whole output is wasted work
+                if (out_cols > (uint32_t)align_up(H, 16u) && c != 64u) eff *= (double)H / out_cols;
+                if (eff > best) { best = eff; bn = c; }
+            }
         }
         if (pl->tune.tc_bn) bn = pl->tune.tc_bn;   // validated when the plan was created
         // Single-CTA alternative for 256-row tiles: two A boxes per stage and two MMAs per
@@ -324,6 +363,8 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
     uint32_t kb_per_split = t.kblocks;
     if (d.split_size) {
         kb_per_split = ceil_div(d.split_size, 64u);
+    } else if (t.pair && !pl->tune.tc_bn) {
+        kb_per_split = ceil_div(t.kblocks, pair_splits);
     } else if (t.num_tiles * 2u <= units && t.kblocks >= 8u) {
         uint32_t want = units / t.num_tiles;
         const uint32_t max_splits = t.kblocks / 4u;      // at least 4 k-blocks (256 of K) per split
@@ -354,7 +395,12 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
         t.stages = stages;
         pl->tc_smem = (size_t)stages * stage_bytes + 1024u + 256u + extra;
     };
-    size_ring(0u);
+    // CTA pairs that store finished outputs do so through shared memory: a lane's own row piece is 16 bytes, half a sector,
+    // and 32 of them per store instruction made the stores the longest part of a tile's epilogue.
+    // Only where the halves of a tile that two warps share are whole 128-byte pieces (a ring stage less otherwise buys nothing:
+    // 192 columns of bf16, 18.0 us staged and 17.2 us direct at 1024 x 2048 x 2048).
+    t.staged = t.pair && t.splits == 1u && ((gate ? bn / 2u : bn) / 2u * dtype_size(d.o_dtype)) % 128u == 0u ? 1u : 0u;
+    size_ring(t.staged ? kTcStagingBytes + 128u : 0u);
     // Split-K folded inside clusters (swapped kernel), on request (tc_fold = 3): the S splits of a tile run as
     // one cluster and add their accumulators up through distributed shared memory, so neither the fp32
     // partial sums nor the fold launch exist.  S is 2, 4 or 8 (each CTA finishes bn / S activation rows, a
@@ -1135,7 +1181,7 @@ int run_impl(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const 
         for (uint32_t i = 0; i < spec->n_dst; ++i) t.dst[i] = spec->dst[i];
         t.rs_rows = spec->rs_rows;
         t.rs_slot = spec->rs_slot;
-        if (t.pair && spec->n_dst > 1u) {
+        if (t.pair && !t.staged && spec->n_dst > 1u) {
             // stores to peers go out as whole 128-byte row segments: one ring stage less, 32 KB of staging
             const uint32_t stage_bytes = 128u * 128u + (t.bn / 2u) * 128u;
             const uint32_t staged_stages = (uint32_t)((kTcMaxSmem - 2048u - kTcStagingBytes - 128u) / stage_bytes);

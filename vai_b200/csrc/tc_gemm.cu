@@ -524,7 +524,15 @@ __device__ __forceinline__ void store_rows16(const TcParams& p, const uint32_t* 
     if (p.partial) {
         // split-K: raw fp32 partial sums, [z][M][N]; epilogue runs in the reduce pass
         float* P = p.partial + (size_t)z * p.M * p.N;
-        if (m < p.M) {
+        const uint32_t j = (GATE ? tb * (bn / 2u) : tb * bn) + c0;
+        if (m < p.M && p.N % 4u == 0u && (!GATE || p.H % 4u == 0u) && j + 16u <= out_cols) {
+            // whole 16-byte pieces of a row: a lane's row is its own, so 4-byte stores would each touch 32 sectors
+#pragma unroll
+            for (uint32_t q = 0; q < 4u; ++q) {
+                reinterpret_cast<uint4*>(P + (size_t)m * p.N + j)[q] = make_uint4(r0[4 * q], r0[4 * q + 1], r0[4 * q + 2], r0[4 * q + 3]);
+                if (GATE) reinterpret_cast<uint4*>(P + (size_t)m * p.N + p.H + j)[q] = make_uint4(r1[4 * q], r1[4 * q + 1], r1[4 * q + 2], r1[4 * q + 3]);
+            }
+        } else if (m < p.M) {
 #pragma unroll
             for (uint32_t c = 0; c < 16u; ++c) {
                 const uint32_t col = c0 + c;
@@ -1312,6 +1320,8 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 //    block, 16-byte chunks XOR-swizzled by the row so that the 32 lanes hit distinct banks
                 uint8_t* mine = staging + (size_t)(warp - 2u) * 4096u + (size_t)lane * 128u;
                 for (uint32_t g = 0; g < seg_cols; g += 16u) {
+                    const ResRaw res_cur = res_next;
+                    if (c0 + g + 16u < c_end) res_issue(p, m, j_seg + g + 16u, out_cols, res_next);      // in flight while this chunk is finished
                     uint32_t r0[16], r1[16];
                     tmem_ld16(t_row + c0 + g, r0);
                     if (GATE) tmem_ld16(t_row + c0 + g + bh, r1);
@@ -1320,7 +1330,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
                     for (int c = 0; c < 16; ++c) { v[c] = __uint_as_float(r0[c]); u[c] = GATE ? __uint_as_float(r1[c]) : 0.0f; }
                     const uint32_t mm = m < p.M ? m : p.M - 1u;          // rows past M compute on a valid row and are not stored
-                    finish_row16<GATE>(p, v, u, mm, j_seg + g, out_cols, 16u);
+                    finish_row16<GATE>(p, v, u, mm, j_seg + g, out_cols, 16u, m < p.M ? &res_cur : nullptr);
                     if (osz == 4u) {
 #pragma unroll
                         for (uint32_t k4 = 0; k4 < 4u; ++k4) {
@@ -1349,19 +1359,28 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 __syncwarp();
                 // 2. eight lanes per row, four rows per store instruction: 4 x 128 contiguous bytes
                 const uint32_t m_base = ta * 2u * TILE_ROWS + rank * TILE_ROWS + q * 32u;
+                const uint32_t member = !GATE && p.grp_t1 != kNoGroup ? (tb >= p.grp_t2 ? 2u : (tb >= p.grp_t1 ? 1u : 0u)) : 0u;
 #pragma unroll
                 for (uint32_t it = 0; it < 8u; ++it) {
                     const uint32_t rr = it * 4u + (lane >> 3), chunk = lane & 7u;
                     const uint4 val = *reinterpret_cast<const uint4*>(staging + (size_t)(warp - 2u) * 4096u + (size_t)rr * 128u + ((chunk ^ (rr & 7u)) * 16u));
-                    if (m_base + rr < p.M) {
-                        uint32_t owner;
-                        size_t row;
-                        output_row(p, m_base + rr, owner, row);
-                        const size_t byte_off = (row * p.ldo + p.col0 + j_seg) * osz + (size_t)chunk * 16u;
-                        for (uint32_t d = 0; d < p.n_dst; ++d)
-                            if (owner == 0xFFFFFFFFu || d == owner)
-                                *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.n_dst == 1u ? p.O : p.dst[d]) + byte_off) = val;
+                    if (m_base + rr >= p.M) continue;
+                    if (!GATE && p.grp_t1 != kNoGroup) {
+                        // a group: members are whole tiles, each a dense matrix of its own width
+                        const uint32_t n1 = p.grp_t1 * bn, n2 = p.grp_t2 == kNoGroup ? p.N : p.grp_t2 * bn;
+                        const uint32_t first = member == 2u ? n2 : (member == 1u ? n1 : 0u);
+                        const uint32_t width = (member == 0u ? n1 : (member == 1u ? n2 : p.N)) - first;
+                        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.dst[member]) +
+                                                  ((size_t)(m_base + rr) * width + (j_seg - first)) * osz + (size_t)chunk * 16u) = val;
+                        continue;
                     }
+                    uint32_t owner;
+                    size_t row;
+                    output_row(p, m_base + rr, owner, row);
+                    const size_t byte_off = (row * p.ldo + p.col0 + j_seg) * osz + (size_t)chunk * 16u;
+                    for (uint32_t d = 0; d < p.n_dst; ++d)
+                        if (owner == 0xFFFFFFFFu || d == owner)
+                            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.n_dst == 1u ? p.O : p.dst[d]) + byte_off) = val;
                 }
                 __syncwarp();
                 c0 += seg_cols;

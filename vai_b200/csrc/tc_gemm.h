@@ -8,7 +8,7 @@
 namespace vaicu {
 
 constexpr size_t kTcMaxSmem = 227u * 1024u;   // opt-in shared memory per CTA on sm_100
-constexpr uint32_t kTcStagingBytes = 8u * 4096u;   // CTA-pair kernel, several destinations: 4 KB per epilogue warp
+constexpr uint32_t kTcStagingBytes = 8u * 4096u;   // CTA-pair kernel: 4 KB per epilogue warp
 
 // How bias / residual are indexed, resolved on the host so the epilogue avoids a
 // 64-bit modulo per element (rule: vAi vai/nodes/linear.h:2333-2338).
@@ -42,7 +42,7 @@ struct TcParams {
     // up to 8 wider destinations at once (its own and its peers' over NVLink).
     uint32_t ldo, col0, n_dst;
     uint32_t staged;       // CTA-pair kernel: finished tiles go through shared memory so that stores to the
-                           // destinations (peers over NVLink) are whole 128-byte row segments
+                           // destination (or destinations, peers over NVLink) are whole 128-byte row segments
     void* dst[8];
     // Row-parallel run (rs_rows > 0): the outputs are partial sums over this GPU's slice of K, and
     // row m belongs to GPU m / rs_rows, which folds the ranks' partials.  Element (m, j) then goes to
