@@ -1,4 +1,4 @@
-"""The streaming decode form (gemv_stream.cu for up to 4 rows, skinny_stream.cu for 5 to 8 on the tensor cores) at the
+"""The streaming decode forms (gemv_stream.cu for one row; skinny_stream.cu for 5 to 8, and for 3 and 4 in 16 bits) at the
 sizes where its geometry can go wrong: K that fills no vector round, one that needs several warps or several register
 loads of activations, fewer columns than blocks, ranges that end inside a stage, more columns than one fold holds."""
 import numpy as np

@@ -44,10 +44,13 @@ template <int N> __device__ __forceinline__ void load_x(const LinearArgs& a, siz
     const uint2* s = reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(a.I) + at);
 #pragma unroll
     for (int q = 0; q < N / 4; ++q) { const uint2 t = s[q]; w[2 * q] = t.x; w[2 * q + 1] = t.y; }
+    if (a.i_dtype == VAICU_DTYPE_F16) {
 #pragma unroll
-    for (int i = 0; i < N / 2; ++i)
-        xf[i] = a.i_dtype == VAICU_DTYPE_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[i]))
-                                             : make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u));
+        for (int i = 0; i < N / 2; ++i) xf[i] = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+    } else {
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) xf[i] = make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u));
+    }
 }
 
 constexpr uint32_t kPartFloats = 2048;           // partial sums held between two folds
@@ -55,16 +58,16 @@ constexpr uint32_t kGemvStreamSmem = kStreamFifoBytes + kPartFloats * 4u;
 
 // XV: 16-byte weight vectors per lane and row.  A block's rows are taken in rounds of 8 / ks, one row per group of ks
 // warps; with a gate a warp alternates between the gate and the value row of its output column.
-template <typename TW, int M, int XV, bool ARGMAX>
+template <typename TW, int XV, bool ARGMAX>
 __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const StreamParams p)
 {
     constexpr int VEC = Vec<TW>::N, PAIRS = VEC / 2;
-    constexpr uint32_t STEP = XV < 4 ? XV : 4;                   // vectors requested, awaited and multiplied together
+    constexpr uint32_t STEP = XV <= 5 ? XV : XV / 2;             // vectors requested, awaited and multiplied together
     constexpr uint32_t STEPS = kStreamDepth / STEP;              // ... and as many such steps under way
     constexpr uint32_t PER_ROW = XV / STEP;
-    static_assert(kStreamDepth % STEP == 0 && XV % STEP == 0, "whole steps");
+    static_assert(XV % STEP == 0, "whole steps");
     extern __shared__ __align__(128) uint8_t smem[];
-    float* part = reinterpret_cast<float*>(smem + kStreamFifoBytes);       // [row][ks][M]
+    float* part = reinterpret_cast<float*>(smem + kStreamFifoBytes);       // [row][ks]
 
     const LinearArgs& a = p.a;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
@@ -104,23 +107,18 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const St
     for (uint32_t i = 0; i + 1u < STEPS; ++i) load_step();
 
     const EpilogueArgs ep = make_epilogue_args(a);
-    float am_best[M];
-    uint32_t am_at[M];
-#pragma unroll
-    for (int m = 0; m < M; ++m) { am_best[m] = kArgmaxLowest; am_at[m] = 0xFFFFFFFFu; }
+    float am_best = kArgmaxLowest;
+    uint32_t am_at = 0xFFFFFFFFu;
 
     dependency_wait();
-    float2 xf[M][XV][PAIRS];
+    float2 xf[XV][PAIRS];
 #pragma unroll
     for (int i = 0; i < XV; ++i) {
         const uint32_t v = v0 + (uint32_t)i * vstep;
+        if (v < nvec) load_x<VEC>(a, (size_t)v * VEC, xf[i]);
+        else
 #pragma unroll
-        for (int m = 0; m < M; ++m) {
-            if (v < nvec) load_x<VEC>(a, (size_t)m * K + (size_t)v * VEC, xf[m][i]);
-            else
-#pragma unroll
-                for (int e = 0; e < PAIRS; ++e) xf[m][i][e] = make_float2(0.0f, 0.0f);
-        }
+            for (int e = 0; e < PAIRS; ++e) xf[i][e] = make_float2(0.0f, 0.0f);
     }
     // bias and residual of this thread's first output, requested ahead of the products
     float early_bias = 0.0f, early_res = 0.0f;
@@ -136,9 +134,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const St
         const uint32_t b1 = b0 + p.batch < u1 ? b0 + p.batch : u1;
         for (uint32_t u = b0 + rg; u < b1; u += RG) {
             for (uint32_t half = 0; half < (gate ? 2u : 1u); ++half) {
-                float2 acc[M][2];
-#pragma unroll
-                for (int m = 0; m < M; ++m) acc[m][0] = acc[m][1] = make_float2(0.0f, 0.0f);
+                float2 acc[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
 #pragma unroll
                 for (uint32_t s = 0; s < PER_ROW; ++s) {
                     load_step();
@@ -152,154 +148,128 @@ __global__ void __launch_bounds__(kStreamThreads, 2) gemv_stream_kernel(const St
                         float2 wf[PAIRS];
                         unpack_w<TW>(wv[i], wf);
 #pragma unroll
-                        for (int m = 0; m < M; ++m)
-#pragma unroll
-                            for (int e = 0; e < PAIRS; ++e) acc[m][e & 1] = __ffma2_rn(wf[e], xf[m][s * STEP + i][e], acc[m][e & 1]);
+                        for (int e = 0; e < PAIRS; ++e) acc[e & 1] = __ffma2_rn(wf[e], xf[s * STEP + i][e], acc[e & 1]);
                     }
                 }
-                float mine = 0.0f;
+                float v = (acc[0].x + acc[0].y) + (acc[1].x + acc[1].y);
 #pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    float v = (acc[m][0].x + acc[m][0].y) + (acc[m][1].x + acc[m][1].y);
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
-                    if (lane == (uint32_t)m) mine = v;
-                }
-                const uint32_t row = (u - b0) + half * p.batch;
-                if (lane < (uint32_t)M) part[((size_t)row * KS + ks) * M + lane] = mine;
+                for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+                if (lane == 0u) part[((u - b0) + half * p.batch) * KS + ks] = v;
             }
         }
         __syncthreads();
         // fold the warps of each row and finish the batch's outputs
         for (uint32_t u = threadIdx.x; u < b1 - b0; u += kStreamThreads) {
             const uint32_t n = b0 + u;
-#pragma unroll
-            for (int m = 0; m < M; ++m) {
-                float v = 0.0f, up = 0.0f;
-                for (uint32_t s = 0; s < KS; ++s) {
-                    v += part[((size_t)u * KS + s) * M + m];
-                    if (gate) up += part[((size_t)(p.batch + u) * KS + s) * M + m];
-                }
-                if (gate) {
-                    const size_t flat = (size_t)m * H + n;
-                    store_from_f32(a.O, a.o_dtype, flat, finish_gated(ep, v, up, n, H, flat));
-                } else if (p.nseg) {
-                    store_segment(p, m, n, v);
-                } else {
-                    const size_t flat = (size_t)m * a.N + n;
-                    const float o = (m == 0 && early && n == u0 + threadIdx.x) ? finish_output_pre(ep, v, early_bias, early_res)
-                                                                               : finish_output(ep, v, flat);
-                    if (!ARGMAX || p.am.write_logits) store_from_f32(a.O, a.o_dtype, flat, o);
-                    // the Argmax node reads the stored logits: compare what the store would hold
-                    if (ARGMAX) argmax_take(round_through(a.o_dtype, o), p.am.index_base + n, am_best[m], am_at[m]);
-                }
+            float v = 0.0f, up = 0.0f;
+            for (uint32_t s = 0; s < KS; ++s) {
+                v += part[u * KS + s];
+                if (gate) up += part[(p.batch + u) * KS + s];
+            }
+            if (gate) {
+                store_from_f32(a.O, a.o_dtype, n, finish_gated(ep, v, up, n, H, n));
+            } else if (p.nseg) {
+                store_segment(p, 0u, n, v);
+            } else {
+                const float o = (early && n == u0 + threadIdx.x) ? finish_output_pre(ep, v, early_bias, early_res) : finish_output(ep, v, n);
+                if (!ARGMAX || p.am.write_logits) store_from_f32(a.O, a.o_dtype, n, o);
+                // the Argmax node reads the stored logits: compare what the store would hold
+                if (ARGMAX) argmax_take(round_through(a.o_dtype, o), p.am.index_base + n, am_best, am_at);
             }
         }
         if (b1 < u1) __syncthreads();            // part is reused by the next batch
     }
 
     if constexpr (ARGMAX) {
-        // the block's candidate per batch row, then the last block to take a ticket folds all of them; nobody waits
-        __shared__ float s_val[kStreamWarps][M];
-        __shared__ uint32_t s_at[kStreamWarps][M];
+        // the block's candidate, then the last block to take a ticket folds all of them; nobody waits
+        __shared__ float s_val[kStreamWarps];
+        __shared__ uint32_t s_at[kStreamWarps];
         __shared__ bool s_last;
-#pragma unroll
-        for (int m = 0; m < M; ++m) {
+        auto warp_best = [&](float& best, uint32_t& at) {
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) {
-                const float ov = __shfl_xor_sync(0xFFFFFFFFu, am_best[m], off);
-                const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, am_at[m], off);
-                argmax_take(ov, oi, am_best[m], am_at[m]);
+                const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, off);
+                const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, at, off);
+                argmax_take(ov, oi, best, at);
             }
-            if (lane == 0u) { s_val[warp][m] = am_best[m]; s_at[warp][m] = am_at[m]; }
+        };
+        warp_best(am_best, am_at);
+        if (lane == 0u) { s_val[warp] = am_best; s_at[warp] = am_at; }
+        __syncthreads();
+        if (threadIdx.x == 0u) {
+            for (uint32_t w = 1; w < kStreamWarps; ++w) argmax_take(s_val[w], s_at[w], am_best, am_at);
+            p.am.block_val[blockIdx.x] = am_best;
+            p.am.block_idx[blockIdx.x] = am_at;
+            __threadfence();                           // the candidate is visible before the ticket
+            s_last = atomicAdd(p.am.count, 1u) == gridDim.x - 1u;
         }
         __syncthreads();
-        if (threadIdx.x < (uint32_t)M) {
+        if (s_last && warp == 0u) {
+            __threadfence();
             float best = kArgmaxLowest;
             uint32_t at = 0xFFFFFFFFu;
-            for (uint32_t w = 0; w < kStreamWarps; ++w) argmax_take(s_val[w][threadIdx.x], s_at[w][threadIdx.x], best, at);
-            p.am.block_val[(size_t)blockIdx.x * M + threadIdx.x] = best;
-            p.am.block_idx[(size_t)blockIdx.x * M + threadIdx.x] = at;
-            __threadfence();                           // candidates visible before the ticket below
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) s_last = atomicAdd(p.am.count, 1u) == gridDim.x - 1u;
-        __syncthreads();
-        if (s_last) {
-            __threadfence();
-            if (warp < (uint32_t)M) {                  // one warp per batch row
-                float best = kArgmaxLowest;
-                uint32_t at = 0xFFFFFFFFu;
-                for (uint32_t b = lane; b < gridDim.x; b += 32u)
-                    argmax_take(__ldcg(p.am.block_val + (size_t)b * M + warp), __ldcg(p.am.block_idx + (size_t)b * M + warp), best, at);
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    const float ov = __shfl_xor_sync(0xFFFFFFFFu, best, off);
-                    const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, at, off);
-                    argmax_take(ov, oi, best, at);
-                }
-                if (lane == 0u) {
-                    p.am.out_idx[warp] = at == 0xFFFFFFFFu ? p.am.index_base : at;   // a row of NaNs: its first column
-                    if (p.am.out_val) p.am.out_val[warp] = best;
-                }
+            for (uint32_t b = lane; b < gridDim.x; b += 32u) argmax_take(__ldcg(p.am.block_val + b), __ldcg(p.am.block_idx + b), best, at);
+            warp_best(best, at);
+            if (lane == 0u) {
+                p.am.out_idx[0] = at == 0xFFFFFFFFu ? p.am.index_base : at;   // a row of NaNs: its first column
+                if (p.am.out_val) p.am.out_val[0] = best;
+                *p.am.count = 0u;                      // ready for the next launch
             }
-            if (threadIdx.x == 0) *p.am.count = 0u;    // ready for the next launch
         }
     }
 }
 
-template <typename TW, int M, int XV, bool ARGMAX>
+template <typename TW, int XV, bool ARGMAX>
 cudaError_t launch_stream_form(const StreamParams& p, int grid, cudaStream_t stream)
 {
-    auto kern = gemv_stream_kernel<TW, M, XV, ARGMAX>;
+    auto kern = gemv_stream_kernel<TW, XV, ARGMAX>;
     static SmemOptIn optin;
     if (cudaError_t e = optin.ensure(kern, (int)kGemvStreamSmem, cudaSharedmemCarveoutMaxShared); e != cudaSuccess) return e;
     return launch_pdl(kern, dim3((unsigned)grid), dim3(kStreamThreads), kGemvStreamSmem, stream, p);
 }
 
-template <typename TW, int M, int XV>
+template <typename TW, int XV>
 cudaError_t launch_stream_one(const StreamParams& p, int grid, cudaStream_t stream)
 {
-    return p.am.out_idx ? launch_stream_form<TW, M, XV, true>(p, grid, stream) : launch_stream_form<TW, M, XV, false>(p, grid, stream);
+    return p.am.out_idx ? launch_stream_form<TW, XV, true>(p, grid, stream) : launch_stream_form<TW, XV, false>(p, grid, stream);
 }
 
 template <typename TW>
 cudaError_t launch_stream_typed(const StreamParams& p, int xv, int grid, cudaStream_t stream)
 {
-    switch (p.a.M * 16u + (uint32_t)xv) {
-    case 16u + 4u: return launch_stream_one<TW, 1, 4>(p, grid, stream);
-    case 16u + 8u: return launch_stream_one<TW, 1, 8>(p, grid, stream);
-    case 32u + 4u: return launch_stream_one<TW, 2, 4>(p, grid, stream);
-    case 48u + 2u: return launch_stream_one<TW, 3, 2>(p, grid, stream);
-    case 64u + 2u: return launch_stream_one<TW, 4, 2>(p, grid, stream);
+    switch (xv) {
+    case 3: return launch_stream_one<TW, 3>(p, grid, stream);
+    case 4: return launch_stream_one<TW, 4>(p, grid, stream);
+    case 5: return launch_stream_one<TW, 5>(p, grid, stream);
+    case 6: return launch_stream_one<TW, 6>(p, grid, stream);
+    case 8: return launch_stream_one<TW, 8>(p, grid, stream);
     default: return cudaErrorInvalidValue;
     }
 }
 
 }  // namespace
 
-// Geometry of the streaming form; false where it does not apply (M > 4, or K too long for the registers that
-// hold the activations: 64 fp32 values a lane for one row, 64 in all for several).
+// Geometry of the streaming form; false where it does not apply: more than one row, or K too long for the registers that
+// hold the activations.  (With 2 to 4 rows the folds of every row's sums take longer than the loads: 2560 x 20480 bf16,
+// 31 / 51 / 61 us against the register form's 21 / 25 / 30.)  The fewest warps per row whose lanes need at most
+// 5 vectors of it, up to 8 where K is too long for that: widths of 3, 4, 5, 6 and 8 vectors leave the usual K (768 to 10240)
+// without a padded vector, and a fold serves several (2560 x 20480: 24.8 us in 4 warps with padding, 18.1 without).
 bool choose_gemv_stream(const LinearArgs& a, int sm_count, GemvStream* out)
 {
     GemvStream c{};
     const uint32_t vec = 16u / dtype_size(a.w_dtype);
     const uint32_t H = a.gate_fuse ? a.N / 2u : a.N;
-    if (a.M == 0u || a.M > 4u || a.K % vec || H == 0u) return false;
+    if (a.M != 1u || a.K % vec || H == 0u) return false;
     const uint32_t nvec = a.K / vec;
-    const uint32_t base_xv = a.M <= 2u ? 4u : 2u;
     uint32_t ks = 1u;
-    while (ks < 8u && (nvec + 32u * ks - 1u) / (32u * ks) > base_xv) ks *= 2u;
+    while (ks < 8u && (nvec + 32u * ks - 1u) / (32u * ks) > 5u) ks *= 2u;
     const uint32_t need = (nvec + 32u * ks - 1u) / (32u * ks);
-    c.xv = (int)base_xv;
-    if (need > base_xv) {
-        if (a.M != 1u || need > 8u) return false;
-        c.xv = 8;
-    }
+    if (need > 8u) return false;
+    c.xv = need <= 3u ? 3 : (need <= 6u ? (int)need : 8);
     c.ks = ks;
     // whole rounds of the warps' row groups between two folds
     const uint32_t rg = kStreamWarps / ks;
-    c.batch = kPartFloats / ((a.gate_fuse ? 2u : 1u) * ks * a.M) / rg * rg;
+    c.batch = kPartFloats / ((a.gate_fuse ? 2u : 1u) * ks) / rg * rg;
     c.grid = (int)(H < (uint32_t)sm_count ? H : (uint32_t)sm_count);
     *out = c;
     return true;

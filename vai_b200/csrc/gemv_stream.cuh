@@ -1,4 +1,4 @@
-// Decode path of Linear, M <= 4, in the form that keeps HBM busy across a chain of layers.
+// Decode path of Linear, one row, in the form that keeps HBM busy across a chain of layers.
 //
 // One persistent block per SM takes a contiguous range of output columns.  Every lane keeps a FIFO of the 16-byte
 // weight vectors that it alone will multiply, in shared memory: it requests them with cp.async, in the order of their
