@@ -12,8 +12,8 @@
 //   * K is split over `k_warps` warps of a block when N alone cannot fill
 //     148 SMs; the fold goes through shared memory, no global scratch;
 //   * blocks are persistent over row groups (grid sized to the SM count).
-// One row takes the streaming form (gemv_stream.cu), 3 and 4 rows in 16 bits that of 5 to 8 rows (skinny_stream.cu); this one
-// keeps the rest of 2 to 8 rows, K beyond 16384, and every geometry that a caller chooses.
+// One row of up to 200 MB of weights takes the streaming form (gemv_stream.cu), 3 and 4 rows in 16 bits that of 5 to 8 rows (skinny_stream.cu); this one
+// keeps larger layers, the rest of 2 to 8 rows, K beyond 16384, and every geometry that a caller chooses.
 #include "common.cuh"
 
 namespace vaicu {
@@ -497,7 +497,9 @@ cudaError_t launch_one(const GemvParams& p, const GemvConfig& cfg, cudaStream_t 
 {
     auto kern = gemv_kernel<TW, M, R, U>;
     static SmemOptIn optin;
-    if (cudaError_t e = optin.ensure(kern, 100 * 1024); e != cudaSuccess) return e;
+    // One row: the loads in flight land in L1, and behind the streaming form (most of the SM as shared memory) there is room for
+    // 28 KB of them instead of 128: the lm_head of a recorded Llama-3.2-1B step lost 55 us that way.
+    if (cudaError_t e = optin.ensure(kern, 100 * 1024, M == 1 ? (int)cudaSharedmemCarveoutMaxL1 : -1); e != cudaSuccess) return e;
     // Programmatic stream serialization: this launch may begin while the kernel ahead
     // of it in the stream drains; gemv_kernel itself waits (dependency_wait) before it
     // reads anything that kernel produced.

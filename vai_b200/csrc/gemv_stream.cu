@@ -249,23 +249,29 @@ cudaError_t launch_stream_typed(const StreamParams& p, int xv, int grid, cudaStr
 
 }  // namespace
 
-// Geometry of the streaming form; false where it does not apply: more than one row, or K too long for the registers that
-// hold the activations.  (With 2 to 4 rows the folds of every row's sums take longer than the loads: 2560 x 20480 bf16,
-// 31 / 51 / 61 us against the register form's 21 / 25 / 30.)  The fewest warps per row whose lanes need at most
-// 5 vectors of it, up to 8 where K is too long for that: widths of 3, 4, 5, 6 and 8 vectors leave the usual K (768 to 10240)
-// without a padded vector, and a fold serves several (2560 x 20480: 24.8 us in 4 warps with padding, 18.1 without).
+// Geometry of the streaming form; false where it does not apply: more than one row (with 2 to 4 the folds of every row's
+// sums take longer than the loads: 2560 x 20480 bf16, 31 / 51 / 61 us against the register form's 21 / 25 / 30), K too long
+// for the registers that hold the activations, or a layer so large that the hand-over no longer counts (the register
+// form keeps 128 KB per SM on their way instead of 96: a 3072 x 128256 head takes 112 us there and 136 us here).
+// The warps per row: the fewest rounds of rows per block, weighed by the vectors of a round and 1.5 for its fold.
 bool choose_gemv_stream(const LinearArgs& a, int sm_count, GemvStream* out)
 {
     GemvStream c{};
-    const uint32_t vec = 16u / dtype_size(a.w_dtype);
+    const uint32_t esz = dtype_size(a.w_dtype), vec = 16u / esz;
     const uint32_t H = a.gate_fuse ? a.N / 2u : a.N;
-    if (a.M != 1u || a.K % vec || H == 0u) return false;
-    const uint32_t nvec = a.K / vec;
-    uint32_t ks = 1u;
-    while (ks < 8u && (nvec + 32u * ks - 1u) / (32u * ks) > 5u) ks *= 2u;
-    const uint32_t need = (nvec + 32u * ks - 1u) / (32u * ks);
-    if (need > 8u) return false;
-    c.xv = need <= 3u ? 3 : (need <= 6u ? (int)need : 8);
+    if (a.M != 1u || a.K % vec || H == 0u || (uint64_t)a.N * a.K * esz > 200000000ull) return false;
+    const uint32_t nvec = a.K / vec, units = (H + (uint32_t)sm_count - 1u) / (uint32_t)sm_count;
+    uint32_t ks = 0u;
+    double best = 1e30;
+    for (uint32_t k = 1u; k <= kStreamWarps; k *= 2u) {
+        const uint32_t need = (nvec + 32u * k - 1u) / (32u * k);
+        if (need > 8u) continue;
+        const int xv = need <= 3u ? 3 : (need <= 6u ? (int)need : 8);        // the widths that are built
+        const uint32_t rg = kStreamWarps / k, rounds = (units + rg - 1u) / rg;
+        const double cost = rounds * (xv + 1.5);
+        if (cost < best) { best = cost; ks = k; c.xv = xv; }
+    }
+    if (!ks) return false;
     c.ks = ks;
     // whole rounds of the warps' row groups between two folds
     const uint32_t rg = kStreamWarps / ks;
