@@ -1,5 +1,6 @@
 """The C++ mirrors of vai::node::Linear and vai::NeuralNet (vai_b200/host/) compiled
-against the C ABI: host logic on CPU, and the nodes end to end on the GPU."""
+against the C ABI: host logic on CPU, and the nodes end to end on the GPU; and the rule on producers of the tcgen05 kernels' ring on a
+CPU model of its barriers."""
 import os
 import subprocess
 
@@ -17,6 +18,7 @@ def _build(name):
     src = os.path.join(CPP, name + ".cpp")
     exe = os.path.join(CPP, name)
     headers = [os.path.join(ROOT, "vai_b200", "host", h) for h in ("linear.h", "net.h", "norm.h", "gated_mul.h", "safetensors.h")]
+    headers.append(os.path.join(ROOT, "vai_b200", "csrc", "tc_ring.h"))
     newest = max(os.path.getmtime(f) for f in [src, _lib.LIB_PATH] + headers)
     if not os.path.exists(exe) or os.path.getmtime(exe) < newest:
         subprocess.run(["g++", "-std=c++20", "-O1", "-Wall", "-o", exe, src, "-L", lib_dir, "-lvaicu",
@@ -24,7 +26,7 @@ def _build(name):
     return exe
 
 
-@pytest.mark.parametrize("name", ["host_linear_test", "host_net_test"])
+@pytest.mark.parametrize("name", ["host_linear_test", "host_net_test", "tc_ring_test"])
 def test_cpp_host_logic(name):
     r = subprocess.run([_build(name)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -35,12 +35,9 @@ namespace {
 constexpr uint32_t BLOCK_K = 64;          // 64 x 2 bytes = one 128-byte swizzle row
 constexpr uint32_t UMMA_K = 16;
 constexpr uint32_t TILE_ROWS = 128;       // UMMA M
-// Warps: 0 producer, 1 MMA issuer, 2-9 epilogue (two per quarter of the TMEM lanes), 10-11 producers.  One thread takes
-// 600-800 cycles to wait for a stage, announce its bytes and issue its two or three copies (170 + 35 + 200 each,
-// measured), longer than the MMAs of most tiles and than HBM needs for a stage, so the k-blocks go round three producers.
-constexpr uint32_t kProducers = 3;
+// Warps: 0 producer, 1 MMA issuer, 2-9 epilogue (two per quarter of the TMEM lanes), 10-11 producers (tc_ring.h).
 constexpr uint32_t kEpiWarps = 8;
-constexpr uint32_t kTcThreads = 32u * (1u + kEpiWarps + kProducers);
+constexpr uint32_t kTcThreads = 32u * (1u + kEpiWarps + kTcProducers);
 constexpr uint32_t kSpinLimit = 1u << 24; // bounded waits (each probe may sleep in hardware)
 
 // ---- PTX wrappers ---------------------------------------------------------
@@ -687,7 +684,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // ---------------- TMA producers, k-block by k-block in turn ----------------
         {
             const bool leader = elect_one();
-            const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps;
+            const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps, producers = tc_producers(stages);
             uint32_t stage = 0, phase = 0, turn = 0;
             bool ok = true;
             // One k-block of one operand into its stage.  "A" sits on the UMMA M axis, "B" on N.
@@ -732,7 +729,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     // follow once it has completed.  (Weights are operand A when swapped, else B.)
                     first = false;
                     const uint32_t npre = (kb1 - kb0 < stages) ? kb1 - kb0 : stages;
-                    for (uint32_t i = me; i < npre; i += kProducers) {        // the ring is empty: no wait needed
+                    for (uint32_t i = me; i < npre; i += producers) {        // the ring is empty: no wait needed
                         if (!leader) continue;
                         mbar_expect_tx(&full_bar[i], tx_bytes);
                         if (SWAP) load_a(i, kb0 + i, ta); else load_b(i, kb0 + i, tb);
@@ -740,12 +737,12 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                     TC_TRACE(2);
                     dependency_wait();
                     TC_TRACE(3);
-                    for (uint32_t i = me; i < npre; i += kProducers) {
+                    for (uint32_t i = me; i < npre; i += producers) {
                         if (!leader) continue;
                         if (SWAP) load_b(i, kb0 + i, tb); else load_a(i, kb0 + i, ta);
                     }
                     kb = kb0 + npre;
-                    turn = npre % kProducers;
+                    turn = npre % producers;
                     stage = npre == stages ? 0u : npre;
                     phase = npre == stages ? 1u : 0u;
                 }
@@ -758,7 +755,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
                             load_b(stage, kb, tb);
                         }
                     }
-                    if (++turn == kProducers) turn = 0;
+                    if (++turn == producers) turn = 0;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
             }
@@ -1160,7 +1157,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // ---------------- TMA producers (both CTAs), k-block by k-block in turn ----------------
         {
             const bool leader = elect_one();
-            const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps;
+            const uint32_t me = warp == 0 ? 0u : warp - 1u - kEpiWarps, producers = tc_producers(stages);
             uint32_t stage = 0, phase = 0, turn = 0;
             bool ok = true;
             bool first = true;
@@ -1190,20 +1187,20 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     // follow once it has completed.
                     first = false;
                     const uint32_t npre = (kb1 - kb0 < stages) ? kb1 - kb0 : stages;
-                    for (uint32_t i = me; i < npre; i += kProducers) {        // the ring is empty: no wait needed
+                    for (uint32_t i = me; i < npre; i += producers) {        // the ring is empty: no wait needed
                         if (!leader) continue;
                         if (rank == 0u) mbar_expect_tx(&full_bar[i], 2u * item_bytes);
                         tma_load_2d_pair(smem + (size_t)i * stage_bytes + a_bytes, mb, map_to_cta(smem_u32(&full_bar[i]), 0u),
                                          (int32_t)((kb0 + i) * BLOCK_K), yb);
                     }
                     dependency_wait();
-                    for (uint32_t i = me; i < npre; i += kProducers)
+                    for (uint32_t i = me; i < npre; i += producers)
                         if (leader) tma_load_2d_pair(smem + (size_t)i * stage_bytes, &tmap_a, map_to_cta(smem_u32(&full_bar[i]), 0u),
                                          (int32_t)((kb0 + i) * BLOCK_K), ya);
                     kb = kb0 + npre;
                     stage = npre == stages ? 0u : npre;
                     phase = npre == stages ? 1u : 0u;
-                    turn = npre % kProducers;
+                    turn = npre % producers;
                 }
                 for (; kb < kb1; ++kb) {
                     if (turn == me) {
@@ -1217,7 +1214,7 @@ tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                             tma_load_2d_pair(sa + a_bytes, mb, bar, kx, yb);
                         }
                     }
-                    if (++turn == kProducers) turn = 0;
+                    if (++turn == producers) turn = 0;
                     if (++stage == stages) { stage = 0; phase ^= 1u; }
                 }
             }

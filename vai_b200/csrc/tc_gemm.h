@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tc_ring.h"
+
 namespace vaicu {
 
 constexpr size_t kTcMaxSmem = 227u * 1024u;   // opt-in shared memory per CTA on sm_100
