@@ -36,7 +36,9 @@ __global__ void __launch_bounds__(kRmsThreads) row_norm_kernel(const RmsParams p
     __shared__ float s_part[kRmsThreads / 32];
     __shared__ float s_part2[kRmsThreads / 32];
     __shared__ float s_inv, s_mean;
-    launch_dependents();
+    // No early launch_dependents(): the Linear kernels request their weights ahead of their own wait, and those may be what
+    // this launch writes, or what a launch ahead of it wrote.  (An early trigger would take 6 us off a sampling head's 150:
+    // norm, 2048 x 128256 lm_head, top 40.)
     dependency_wait();
     for (uint32_t row = blockIdx.x; row < p.rows; row += gridDim.x) {
         const size_t base = (size_t)row * p.feat;

@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(kPartThreads) topk_slice_kernel(const TopkPara
 {
     const uint32_t row = blockIdx.y, g = blockIdx.x, G = gridDim.x, tid = threadIdx.x;
     __shared__ Kept s;
-    launch_dependents();
     dependency_wait();
+    launch_dependents();         // behind the wait: a Linear after this may request weights that a launch ahead has written
     const uint32_t slice = (p.N + G - 1u) / G;
     const uint32_t s0 = g * slice, s1 = (s0 + slice < p.N) ? s0 + slice : p.N;
     float v[kList];
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(kPartThreads) topk_merge_kernel(const TopkPara
 {
     const uint32_t row = blockIdx.x, tid = threadIdx.x, G = p.N;
     __shared__ Kept s;
-    launch_dependents();
     dependency_wait();
+    launch_dependents();         // behind the wait: a Linear after this may request weights that a launch ahead has written
     const uint2* lists = p.cand_in + (size_t)row * p.row_stride;
     // the bound: the first entries of the lists, k of them where the lists are that long, at most 256: one per thread
     const uint32_t even = (p.k + G - 1u) / G, ahead = even < p.list_len ? even : p.list_len;
