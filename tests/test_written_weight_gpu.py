@@ -63,3 +63,28 @@ def test_wired_norm(M, device):
         # a weight at the edge of a bf16 rounding may fall on its other side, 2^-8 of up to 4, times an activation of up to 4:
         # four of them in one output.  Outputs are of the order of 45; a weight read too early is the last call's.
         assert_close(got, (torch.from_numpy(x).double() @ _normed(torch.from_numpy(raw)).t()).numpy(), (1e-4, 0.25), f"M={M} call {i}")
+
+
+@pytest.mark.parametrize("M,argmax", [(1, False), (1, True), (6, False), (40, False), (200, False)])
+def test_wired_linear(M, argmax, device):
+    """The weight is another Linear's output: that kernel lets its successor start early."""
+    net = NeuralNet(w_default_dtype=Dtype.BF16)
+    inner, lin = nodes.LinearNode(in_dim=K, out_dim=K), nodes.LinearNode(in_dim=K, out_dim=N)
+    inner.set_o_dtype(Dtype.BF16)
+    rng = np.random.default_rng(M)
+    inner["weight"] = Tensor.from_numpy(np.eye(K, dtype=np.float32)[::-1].copy(), dtype=Dtype.BF16)      # reverses the columns: exact
+    if argmax:
+        net.input("x") - lin - nodes.ArgmaxNode() - net.output("y")
+    else:
+        net.input("x") - lin - net.output("y")
+    net.input("w") - inner
+    inner - "weight" / lin
+    for i in range(3):
+        x = torch.from_numpy(rng.standard_normal((M, K), dtype=np.float32)).bfloat16()
+        raw = torch.from_numpy(rng.standard_normal((N, K), dtype=np.float32)).bfloat16()
+        got = net(x=Tensor.from_numpy(x.float().numpy()), w=Tensor.from_numpy(raw.float().numpy()))
+        want = x.double() @ raw.double().flip(1).t()
+        if argmax:
+            np.testing.assert_array_equal(got.to_u32().reshape(-1), want.argmax(-1).numpy())
+        else:
+            assert_close(got.to_numpy(), want.numpy(), (1e-4, 1e-3), f"M={M} call {i}")      # fp32 sums of exact products

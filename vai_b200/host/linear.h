@@ -251,12 +251,13 @@ public:
     bool gateFused() const { return gate_; }
     void resetFusion() override { gate_ = false; argmaxReader_ = nullptr; launchTaken_ = false; group_.clear(); groupWork_ = nullptr; }
 
+    bool weightComputed() const { return links().count("weight") != 0; }
     // Plain (nothing after the dot product) on the weight-streaming kernel, or on the swapped
     // tensor-core kernel with a whole number of weight tiles: vaicu_linear_run_group can serve
     // this node together with siblings over the same activations.
     std::string groupKey() const override
     {
-        if (!plan_ || hasBias() || config_.acceptResidual || config_.epilogue != vai::Epilogue::None || gate_ ||
+        if (!plan_ || weightComputed() || hasBias() || config_.acceptResidual || config_.epilogue != vai::Epilogue::None || gate_ ||
             config_.scalarScale != 1.0f || argmaxReader_ || config_.splitSize)
             return {};
         const bool ok = info_.kernel == VAICU_KERNEL_GEMV || (info_.kernel == VAICU_KERNEL_TC_SKINNY && config_.outDim % 128u == 0) ||
@@ -353,6 +354,9 @@ public:
     void run(vaicu_stream_t stream) override
     {
         if (!plan_) throw std::logic_error("Linear::run before prepare");
+        // A weight that a node computes: the kernels request weights before the launch ahead has completed, so a plain
+        // stream operation (on bytes that this run overwrites) goes in between.
+        if (weightComputed()) check(vaicu_memset((*this)["out0"].devicePtr(), 0, 2, stream), "vaicu_memset");
         if (launchTaken_) return;      // the Argmax behind this node, or the group's first member, launches for it
         if (!group_.empty()) {
             vaicu_linear_plan* plans[3];

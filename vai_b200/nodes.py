@@ -170,10 +170,16 @@ class LinearNode(Node):
         r = self["residual"].ptr if self.accept_residual else None
         ws = self["partial"].ptr if self["partial"].valid_shape() else None
         run = dev.lib.vaicu_linear_run
+        # A weight that a node computes: the kernels request weights before the launch ahead has completed, so a plain
+        # stream operation (on bytes that this run overwrites) goes in between.
+        order = dev.lib.vaicu_memset if self._weight_computed() else None
+        order_bytes = min(4, self["out0"].nbytes())
 
         node = self
 
         def launch(stream):
+            if order is not None:
+                _lib.check(order(o, 0, order_bytes, stream), "vaicu_memset")
             if node._launch_taken:        # the Argmax behind this node launches the fused kernel
                 return
             _lib.check(run(plan, stream, x, w, b, r, o, ws), "vaicu_linear_run")
@@ -182,6 +188,10 @@ class LinearNode(Node):
         self._launch = launch
         return launch
 
+    def _weight_computed(self):
+        from .engine import InputNode
+        return "weight" in self.links and not isinstance(self.links["weight"][0], InputNode)
+
     def groupable(self):
         """Plain (nothing after the dot product) and on the weight-streaming kernel, or on a
         tensor-core kernel with a whole number of weight tiles: may share one launch with
@@ -189,6 +199,8 @@ class LinearNode(Node):
         if self.info is None or self.has_bias() or self.accept_residual or self.epilogue != Epilogue.NONE:
             return False
         if self.gate_fuse or self.scalar_scale != 1.0 or self._argmax_reader is not None or self.split_size:
+            return False
+        if self._weight_computed():
             return False
         if self.info.kernel == KERNEL_TC_GEMM:      # CTA pairs: whole 256-column tiles, 16-bit activations (no cast pass)
             return self.out_dim % 256 == 0 and self["in0"].dtype != Dtype.F32
