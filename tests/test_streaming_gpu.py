@@ -1,13 +1,16 @@
-"""The streaming decode forms (gemv_stream.cu for one row; skinny_stream.cu for 5 to 8, and for 3 and 4 in 16 bits) at the
-sizes where its geometry can go wrong: K that fills no vector round, one that needs several warps or several register
+"""The streaming decode forms (gemv_stream.cu for one row, skinny_stream.cu for 5 to 8) at the sizes where their
+geometry can go wrong: K that fills no vector round, one that needs several warps or several register
 loads of activations, fewer columns than blocks, ranges that end inside a stage, more columns than one fold holds."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 from gpu_util import out_tol, run_linear, seen
 from linear_check import assert_close
 
 from oracle import linear_oracle as orc
-from vai_b200 import Dtype, Epilogue, NeuralNet, Tensor, nodes
+from vai_b200 import Dtype, Epilogue, NeuralNet, Tensor, _lib, nodes
 
 pytestmark = pytest.mark.gpu
 
@@ -86,3 +89,27 @@ def test_streaming_epilogues_and_orders(device):
             got, want, _ = run_linear(x[:M].copy(), w, b, r[:M].copy(), w_dtype="bf16", epilogue=ep.name,
                                       residual_order="BEFORE_EPILOGUE", scalar_scale=0.25)
             assert_close(got, want, (1e-4, 1e-5), f"{ep.name} M={M}")
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("kernel", [nodes.KERNEL_AUTO, nodes.KERNEL_GEMV])
+@pytest.mark.parametrize("dt", [Dtype.F16, Dtype.BF16])
+def test_fused_argmax_stores_the_logits_of_a_run(M, kernel, dt, device):
+    """vaicu_linear_run_argmax gives what vaicu_linear_run and an Argmax give: the same logits, to the bit, on the plan's kernel."""
+    K, N, lib = 2560, 3000, device.lib
+    g = torch.Generator(device="cuda").manual_seed(M)
+    tdt = torch.float16 if dt == Dtype.F16 else torch.bfloat16
+    x, w = (torch.randn(s, K, device="cuda", generator=g).to(tdt) for s in (M, N))
+    d = _lib.LinearDesc(M=M, N=N, K=K, i_dtype=int(dt), w_dtype=int(dt), o_dtype=int(dt), b_dtype=int(Dtype.NONE), scalar_scale=1.0)
+    plan, need = ctypes.c_void_p(), ctypes.c_size_t()
+    tuning = _lib.LinearTuning(kernel=kernel)
+    _lib.check(lib.vaicu_linear_plan_create_tuned(device.handle, ctypes.byref(d), ctypes.byref(tuning), ctypes.byref(plan)), "plan")
+    _lib.check(lib.vaicu_linear_argmax_workspace_bytes(plan, ctypes.byref(need)), "workspace")
+    ws, pick = torch.zeros(need.value, dtype=torch.uint8, device="cuda"), torch.zeros(M, dtype=torch.int32, device="cuda")
+    alone, fused = torch.zeros(M, N, dtype=tdt, device="cuda"), torch.zeros(M, N, dtype=tdt, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.vaicu_linear_run(plan, s, x.data_ptr(), w.data_ptr(), None, None, alone.data_ptr(), None), "run")
+    _lib.check(lib.vaicu_linear_run_argmax(plan, s, x.data_ptr(), w.data_ptr(), None, None, fused.data_ptr(), ws.data_ptr(), 0, None,
+                                           pick.data_ptr()), "run_argmax")
+    assert torch.equal(alone, fused)
+    lib.vaicu_linear_plan_destroy(plan)

@@ -173,7 +173,6 @@ struct GemvStream { int xv; uint32_t ks, batch; int grid; };
 struct GemvConfig {
     int rows_per_warp; int k_warps; int grid; size_t smem; int vectorized; int unroll; int plain_launch;
     int streaming; GemvStream stream;
-    int tensor; int sm_count;      // skinny_stream.cu (not with an Argmax)
 };
 bool choose_gemv_stream(const LinearArgs& a, int sm_count, GemvStream* out);
 cudaError_t launch_gemv_stream(const LinearArgs& a, const GemvConfig& cfg, uint32_t nseg, const uint32_t* rows, const void* const* w,

@@ -12,8 +12,8 @@
 //   * K is split over `k_warps` warps of a block when N alone cannot fill
 //     148 SMs; the fold goes through shared memory, no global scratch;
 //   * blocks are persistent over row groups (grid sized to the SM count).
-// One row of up to 200 MB of weights takes the streaming form (gemv_stream.cu), 3 and 4 rows in 16 bits that of 5 to 8 rows (skinny_stream.cu); this one
-// keeps larger layers, the rest of 2 to 8 rows, K beyond 16384, and every geometry that a caller chooses.
+// One row of up to 200 MB of weights takes the streaming form (gemv_stream.cu); this one keeps larger layers, 2 to 8 rows,
+// K beyond 16384, and every geometry that a caller chooses.
 #include "common.cuh"
 
 namespace vaicu {
@@ -567,11 +567,6 @@ GemvConfig choose_gemv(const LinearArgs& a, int sm_count, bool ptrs_aligned16, c
         c.grid = c.stream.grid;
         return c;
     }
-    // 3 and 4 rows in 16 bits throughout: products of such operands are exact on the tensor cores and the result is rounded
-    // to 16 bits anyway, so they share the form of 5 to 8 rows (2560 x 20480 bf16: 25 / 30 us here, 21 us there).
-    c.sm_count = sm_count;
-    c.tensor = c.vectorized && !tuned && a.M >= 3u && a.M <= 4u && a.w_dtype != VAICU_DTYPE_F32 && a.i_dtype == a.w_dtype &&
-               a.o_dtype != VAICU_DTYPE_F32;
     if (!c.vectorized) {
         c.rows_per_warp = 1; c.k_warps = 1; c.smem = 0;
         c.grid = (int)((H + kWarps - 1u) / kWarps);
@@ -654,7 +649,6 @@ cudaError_t launch_gemv_group(const LinearArgs& a, const GemvConfig& cfg, uint32
                               const void* const* w, void* const* o, cudaStream_t stream)
 {
     if (nseg < 2u || nseg > 3u || !cfg.vectorized || a.gate_fuse) return cudaErrorInvalidValue;
-    if (cfg.tensor) return launch_skinny_stream(a, cfg.sm_count, nseg, rows, w, o, stream);
     if (cfg.streaming) return launch_gemv_stream(a, cfg, nseg, rows, w, o, nullptr, stream);
     GemvParams p{};
     p.a = a;
@@ -689,7 +683,6 @@ cudaError_t launch_gemv_group(const LinearArgs& a, const GemvConfig& cfg, uint32
 cudaError_t launch_gemv(const LinearArgs& a, const GemvConfig& cfg, cudaStream_t stream, const GemvArgmax* argmax)
 {
     if (argmax && (!cfg.vectorized || a.gate_fuse)) return cudaErrorInvalidValue;
-    if (cfg.tensor && !argmax) return launch_skinny_stream(a, cfg.sm_count, 0u, nullptr, nullptr, nullptr, stream);
     if (cfg.streaming) return launch_gemv_stream(a, cfg, 0u, nullptr, nullptr, nullptr, argmax, stream);
     GemvParams p{};
     p.a = a;

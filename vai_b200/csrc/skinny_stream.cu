@@ -1,5 +1,5 @@
-// Linear with 5 to 8 rows of activations (3 and 4 in 16 bits throughout) and 16-bit weights: the streaming decode form (gemv_stream.cuh) with its
-// dot products on mma.sync.
+// Linear with 5 to 8 rows of activations and 16-bit weights: the streaming decode form (gemv_stream.cuh) with its dot
+// products on mma.sync.
 //
 // At these sizes the layer is still bound by the bytes of its weights (8 rows: 8 MACs per weight), but one
 // FMA per weight and row is more than the FMA units deliver at HBM speed, and the tcgen05 kernel pays for its
