@@ -29,7 +29,7 @@ def test_streaming_plain(M, K, N, dt, device):
     x, w, b, r = _draw(M, K, N)
     got, want, node = run_linear(x, w, b, r, i_dtype=dt[0], w_dtype=dt[1], o_dtype=dt[2], epilogue="GELU", scalar_scale=0.5)
     assert node.info.kernel == (nodes.KERNEL_GEMV if M <= 4 else nodes.KERNEL_TC_SKINNY)
-    assert node.info.launches == 1
+    assert node.info.launches == 1 or M > 4
     # fp32 sums; the error-function polynomial of the GELU is good to 1.5e-7 of its argument
     assert_close(got, want, out_tol(dt[2]), f"{M}x{K}x{N} {dt}")
 
@@ -113,3 +113,27 @@ def test_fused_argmax_stores_the_logits_of_a_run(M, kernel, dt, device):
                                            pick.data_ptr()), "run_argmax")
     assert torch.equal(alone, fused)
     lib.vaicu_linear_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("K,N,gate,streamed", [
+    (2048, 8192, False, True), (2048, 148 * 96, False, True), (2048, 148 * 96 + 1, False, False), (1536, 148 * 96 + 1, False, True),
+    (768, 148 * 112 + 1, False, False), (2048, 128256, False, False), (64, 16384, False, False), (2048, 148 * 96, True, True),
+    (2048, 148 * 96 + 2, True, False), (8192, 2048, False, True), (8192, 148 * 16 + 1, False, False), (8192, 148 * 7, False, False),
+    (8200, 2048, False, False), (12288, 300, False, False)])
+def test_five_to_eight_rows_choice(K, N, gate, streamed, device):
+    """Which layers of 5 to 8 rows take the one-launch form: fp32 activations, so the tcgen05 kernel has a cast ahead of it."""
+    d = _lib.LinearDesc(M=8, N=N, K=K, i_dtype=int(Dtype.F32), w_dtype=int(Dtype.BF16), o_dtype=int(Dtype.F32), b_dtype=int(Dtype.NONE),
+                        scalar_scale=1.0, gate_fuse=int(gate))
+    plan, info = ctypes.c_void_p(), _lib.LinearInfo()
+    _lib.check(device.lib.vaicu_linear_plan_create(device.handle, ctypes.byref(d), ctypes.byref(plan)), "plan")
+    _lib.check(device.lib.vaicu_linear_plan_info(plan, ctypes.byref(info)), "info")
+    assert (info.launches == 1) == streamed
+    device.lib.vaicu_linear_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("M", [5, 8])
+@pytest.mark.parametrize("K,N", [(1536, 148 * 112), (1536, 148 * 112 + 1), (8192, 148 * 16), (8192, 148 * 16 + 8), (4096, 14200)])
+def test_five_to_eight_rows_on_both_sides_of_the_choice(M, K, N, device):
+    x, w, b, r = _draw(M, K, N)
+    got, want, _ = run_linear(x, w, b, r, w_dtype="bf16")
+    assert_close(got, want, (1e-4, 1e-5), f"{M}x{K}x{N}")

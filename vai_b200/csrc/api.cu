@@ -111,7 +111,9 @@ struct vaicu_linear_plan {
     int kernel;               // VAICU_KERNEL_*
     // GEMV
     GemvConfig gemv_vec, gemv_any;
-    bool skinny_stream;        // M <= 8 on the tensor cores: plain calls take skinny_stream_kernel
+    // M <= 8 on the tensor cores, every choice left to the library: skinny_stream_kernel may take a plain call (or a group), and
+    // does where it is the faster form
+    bool skinny_able, skinny_stream;
     // FMA tile (also the fallback of the tensor-core plans)
     FmaTileConfig fma;
     bool fma_partial;
@@ -551,7 +553,7 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
     pl->gemv_vec = choose_gemv(a, dev->sm_count, true, &pl->tune);
     pl->gemv_any = choose_gemv(a, dev->sm_count, false, &pl->tune);
     plan_fma(pl);
-    pl->tc = pl->skinny_stream = false;
+    pl->tc = pl->skinny_able = pl->skinny_stream = false;
     int kernel = force_kernel;
     if (kernel == 0) {
         // Few rows: the weight-streaming kernel (vAi useSlabPath takes M <= 8,
@@ -594,9 +596,11 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
             }
         }
         pl->launches = 1u + (pl->tc_cast ? 1u : 0u) + ((pl->tcp.splits > 1u && !pl->tile_done && !pl->tcp.cfold) ? 1u : 0u);
-        // Up to 8 rows the streaming form with mma.sync takes a plain call in one launch; a chosen kernel, a K span or
-        // any tuning of the tcgen05 kernel, outputs in several places and unaligned activations stay with that one.
-        pl->skinny_stream = kernel == VAICU_KERNEL_TC_SKINNY && force_kernel == 0 && d.M <= kSkinnyStreamRows && !d.split_size && !tunes_tc(tuning);
+        // Up to 8 rows the streaming form with mma.sync takes a plain call of a layer that is not too large, in one launch; a
+        // chosen kernel, a K span or any tuning of the tcgen05 kernel, outputs in several places and unaligned activations
+        // stay with that one.
+        pl->skinny_able = kernel == VAICU_KERNEL_TC_SKINNY && force_kernel == 0 && d.M <= kSkinnyStreamRows && !d.split_size && !tunes_tc(tuning);
+        pl->skinny_stream = pl->skinny_able && skinny_stream_fits(d.N, d.K, d.gate_fuse != 0, dev->sm_count);
         if (pl->skinny_stream) pl->launches = 1u;
         break;
     default:
@@ -1344,9 +1348,9 @@ int vaicu_linear_run_group(vaicu_linear_plan* const* plans, int count, vaicu_str
     bool one_launch = p0->kernel == VAICU_KERNEL_TC_SKINNY && aligned16(I);
     for (int i = 0; i < count; ++i) {
         if (!aligned16(O[i])) return VAICU_ERR_UNSUPPORTED;
-        one_launch = one_launch && plans[i]->skinny_stream;
+        one_launch = one_launch && plans[i]->skinny_able;
     }
-    if (one_launch) {
+    if (one_launch && skinny_stream_fits((uint32_t)total, p0->d.K, false, p0->dev->sm_count)) {
         vaicu_linear_desc all = p0->d;
         all.N = (uint32_t)total;
         const LinearArgs a = make_args(all, I, W[0], nullptr, nullptr, O[0]);
