@@ -115,7 +115,7 @@ typedef struct vaicu_linear_info {
     int32_t  kernel;         /* VAICU_KERNEL_*                                  */
     uint32_t split_count;    /* K splits (1 = none)                             */
     uint32_t tile_m, tile_n; /* CTA tile (rows of O, columns of O); 0 for GEMV  */
-    uint32_t launches;       /* kernels one vaicu_linear_run() enqueues         */
+    uint32_t launches;       /* kernels one vaicu_linear_run() enqueues (on the plan's own kernel) */
     size_t   workspace_bytes;
 } vaicu_linear_info;
 
@@ -278,7 +278,9 @@ VAICU_API int vaicu_linear_run_argmax(vaicu_linear_plan* plan, vaicu_stream_t st
  * must be plain (no bias, epilogue, residual, scale or gate), share M, K and dtypes, and
  * resolve to the same kernel, with 16-byte aligned operands:
  *   - the weight-streaming kernel: one launch, no workspace;
- *   - the swapped tensor-core kernel (8 < M <= 128), every N a multiple of 128: one GEMM
+ *   - M = 5..8 with 16-bit weights, every N a multiple of 128, up to some 70 MB of weights in all: one launch of
+ *     the tensor-core form of the weight-streaming kernel, no workspace;
+ *   - the swapped tensor-core kernel (M <= 128 otherwise), every N a multiple of 128: one GEMM
  *     launch that leaves fp32 partial sums of all members plus one fold that stores the
  *     members' outputs (where three runs would be three GEMMs and three folds); fp32
  *     activations are rounded to the weights' type once.  Needs `workspace` of

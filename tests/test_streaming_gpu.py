@@ -43,25 +43,78 @@ def test_streaming_gate(M, K, H, w_dtype, device):
     assert_close(got, want, (1e-4, 1e-5), f"gate {M}x{K}x{H} {w_dtype}")
 
 
-@pytest.mark.parametrize("M", [1, 4, 8])
+@pytest.mark.parametrize("M", [1, 3, 4, 8])
 @pytest.mark.parametrize("K,widths", [(768, (128, 256, 128)), (2560, (2048, 1024, 1024)), (520, (128, 128))])
-def test_streaming_group(M, K, widths, device):
+@pytest.mark.parametrize("io", ["f32", "bf16"])
+def test_streaming_group(M, K, widths, io, device):
     """Sibling Linears of one input in one launch: ranges and stages that straddle the members."""
+    _group(M, K, widths, io, 1)
+
+
+@pytest.mark.parametrize("K,widths,tuning,launches", [(4096, (8192, 8192), None, 2), (2560, (1024, 1024), dict(tc_splits=1), 2),
+                                                      (8200, (256, 128), None, 2), (4096, (8192, 4096), None, 1)])
+def test_group_of_eight_rows_counts_its_launches(K, widths, tuning, launches, device):
+    """GEMM and fold where the members together are too large for one launch, too deep, or tuned."""
+    _group(8, K, widths, "bf16", launches, tuning)
+
+
+def _group(M, K, widths, io, launches, tuning=None):
     rng = np.random.default_rng(K + M)
     x = rng.standard_normal((M, K)).astype(np.float32)
     ws = [(rng.standard_normal((n, K)) / np.sqrt(K)).astype(np.float32) for n in widths]
-    net = NeuralNet(w_default_dtype=Dtype.BF16, guard_bytes=512)
+    dt = Dtype.BF16 if io == "bf16" else Dtype.F32
+    net = NeuralNet(w_default_dtype=Dtype.BF16, o_default_dtype=dt, guard_bytes=512)
     src = net.input("x")
     for i, w in enumerate(ws):
-        lin = nodes.LinearNode(in_dim=K, out_dim=w.shape[0])
+        lin = nodes.LinearNode(in_dim=K, out_dim=w.shape[0], tuning=tuning)
         lin["weight"] = Tensor.from_numpy(w, dtype=Dtype.BF16)
         src - lin - net.output(f"y{i}")
-    out = net(Tensor.from_numpy(x))
-    assert next(iter(net._recordings.values())).kernel_launches == 1
+    out = net(Tensor.from_numpy(x, dtype=dt))
+    assert next(iter(net._recordings.values())).kernel_launches == launches
     net.pool.check_guards()
-    xs = x if M <= 4 else seen(x, Dtype.BF16)
+    xs = x if M <= 4 and io == "f32" else seen(x, Dtype.BF16)
     for i, w in enumerate(ws):
-        assert_close(out[f"y{i}"].to_numpy(), orc.linear_f64(xs, seen(w, Dtype.BF16)), (1e-4, 1e-5), f"member {i}")
+        assert_close(out[f"y{i}"].to_numpy(), orc.linear_f64(xs, seen(w, Dtype.BF16)), out_tol(io), f"member {i}")
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("M", [5, 8])
+def test_unaligned_fp32_activations_of_five_to_eight_rows(M, grouped, device):
+    """Activations at any fp32 element: the same launch and the same bits as aligned ones, without a workspace."""
+    K, widths, lib = 2056, (256, 384), device.lib
+    g = torch.Generator(device="cuda").manual_seed(M)
+    held = torch.randn(M * K + 4, device="cuda", generator=g)
+    x = held[1:1 + M * K]
+    same = x.clone()
+    plans, ws, outs = [], [], []
+    for n in widths:
+        d = _lib.LinearDesc(M=M, N=n, K=K, i_dtype=int(Dtype.F32), w_dtype=int(Dtype.BF16), o_dtype=int(Dtype.F32), b_dtype=int(Dtype.NONE),
+                            scalar_scale=1.0)
+        h, info = ctypes.c_void_p(), _lib.LinearInfo()
+        _lib.check(lib.vaicu_linear_plan_create(device.handle, ctypes.byref(d), ctypes.byref(h)), "plan")
+        _lib.check(lib.vaicu_linear_plan_info(h, ctypes.byref(info)), "info")
+        plans.append(h)
+        ws.append(torch.randn(n, K, device="cuda", generator=g).bfloat16())
+        outs.append([torch.zeros(M, n, device="cuda") for _ in range(2)])
+        work = torch.empty(max(info.workspace_bytes, 256), dtype=torch.uint8, device="cuda")
+    s = torch.cuda.current_stream().cuda_stream
+    for k, act in enumerate((x, same)):
+        if grouped:
+            need = ctypes.c_size_t(1)
+            arr = (ctypes.c_void_p * 2)(*plans)
+            _lib.check(lib.vaicu_linear_group_workspace_bytes(arr, 2, ctypes.byref(need)), "group")
+            assert need.value == 0
+            _lib.check(lib.vaicu_linear_run_group(arr, 2, s, act.data_ptr(), (ctypes.c_void_p * 2)(*[w.data_ptr() for w in ws]),
+                                                  (ctypes.c_void_p * 2)(*[o[k].data_ptr() for o in outs]), None), "run_group")
+        else:
+            for h, w, o in zip(plans, ws, outs):
+                _lib.check(lib.vaicu_linear_run(h, s, act.data_ptr(), w.data_ptr(), None, None, o[k].data_ptr(), work.data_ptr()), "run")
+    for w, o in zip(ws, outs):
+        assert torch.equal(o[0], o[1])
+        want = same.reshape(M, K).bfloat16().double() @ w.double().t()
+        assert_close(o[0].cpu().numpy(), want.cpu().numpy(), (1e-4, 1e-3), "unaligned")
+    for h in plans:
+        lib.vaicu_linear_plan_destroy(h)
 
 
 @pytest.mark.parametrize("M", [1, 2, 4])

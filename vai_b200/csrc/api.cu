@@ -597,8 +597,7 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
         }
         pl->launches = 1u + (pl->tc_cast ? 1u : 0u) + ((pl->tcp.splits > 1u && !pl->tile_done && !pl->tcp.cfold) ? 1u : 0u);
         // Up to 8 rows the streaming form with mma.sync takes a plain call of a layer that is not too large, in one launch; a
-        // chosen kernel, a K span or any tuning of the tcgen05 kernel, outputs in several places and unaligned activations
-        // stay with that one.
+        // chosen kernel, a K span or any tuning of the tcgen05 kernel and outputs in several places stay with that one.
         pl->skinny_able = kernel == VAICU_KERNEL_TC_SKINNY && force_kernel == 0 && d.M <= kSkinnyStreamRows && !d.split_size && !tunes_tc(tuning);
         pl->skinny_stream = pl->skinny_able && skinny_stream_fits(d.N, d.K, d.gate_fuse != 0, dev->sm_count);
         if (pl->skinny_stream) pl->launches = 1u;
@@ -1134,7 +1133,7 @@ int run_impl(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const 
     }
     pl->last_kernel = pl->kernel;
     pl->last_vectorized = 1;
-    if (pl->skinny_stream && !spec && aligned16(I)) {
+    if (pl->skinny_stream && !spec) {
         VAICU_CUDA(launch_skinny_stream(a, pl->dev->sm_count, 0u, nullptr, nullptr, nullptr, s));
         return VAICU_OK;
     }
@@ -1258,6 +1257,17 @@ int group_members_ok(vaicu_linear_plan* const* plans, int count)
     return VAICU_OK;
 }
 
+// Up to 8 rows: the members side by side on skinny_stream_kernel, in one launch without a workspace.
+bool group_streams(vaicu_linear_plan* const* plans, int count)
+{
+    uint32_t total = 0;
+    for (int i = 0; i < count; ++i) {
+        if (!plans[i]->skinny_able) return false;
+        total += plans[i]->d.N;
+    }
+    return skinny_stream_fits(total, plans[0]->d.K, false, plans[0]->dev->sm_count);
+}
+
 // The cached state of a tensor-core group, (re)built when the members change.
 int group_state(vaicu_linear_plan* const* plans, int count, GroupState** out)
 {
@@ -1308,7 +1318,7 @@ int vaicu_linear_group_workspace_bytes(vaicu_linear_plan* const* plans, int coun
     int rc = group_members_ok(plans, count);
     if (rc != VAICU_OK) return rc;
     *out_bytes = 0;
-    if (plans[0]->kernel == VAICU_KERNEL_GEMV) return VAICU_OK;
+    if (plans[0]->kernel == VAICU_KERNEL_GEMV || group_streams(plans, count)) return VAICU_OK;
     GroupState* g = nullptr;
     rc = group_state(plans, count, &g);
     if (rc != VAICU_OK) return rc;
@@ -1344,13 +1354,11 @@ int vaicu_linear_run_group(vaicu_linear_plan* const* plans, int count, vaicu_str
         VAICU_CUDA(launch_gemv_group(a, cfg, (uint32_t)count, rows, W, O, s));
         return VAICU_OK;
     }
-    // swapped tensor-core kernel: one launch leaves the partial sums of all members, one fold stores the outputs
-    bool one_launch = p0->kernel == VAICU_KERNEL_TC_SKINNY && aligned16(I);
-    for (int i = 0; i < count; ++i) {
+    for (int i = 0; i < count; ++i)
         if (!aligned16(O[i])) return VAICU_ERR_UNSUPPORTED;
-        one_launch = one_launch && plans[i]->skinny_able;
-    }
-    if (one_launch && skinny_stream_fits((uint32_t)total, p0->d.K, false, p0->dev->sm_count)) {
+    if (group_streams(plans, count)) {
+        if (p0->d.i_dtype != VAICU_DTYPE_F32 && !aligned16(I)) return VAICU_ERR_UNSUPPORTED;
+        if (reinterpret_cast<uintptr_t>(I) & (dtype_size(p0->d.i_dtype) - 1u)) return VAICU_ERR_ALIGNMENT;
         vaicu_linear_desc all = p0->d;
         all.N = (uint32_t)total;
         const LinearArgs a = make_args(all, I, W[0], nullptr, nullptr, O[0]);
@@ -1392,6 +1400,7 @@ int vaicu_linear_run_group(vaicu_linear_plan* const* plans, int count, vaicu_str
         for (int i = 0; i < count; ++i) { plans[i]->last_kernel = VAICU_KERNEL_TC_GEMM; plans[i]->last_vectorized = 1; }
         return VAICU_OK;
     }
+    // swapped tensor-core kernel: one launch leaves the partial sums of all members, one fold stores the outputs
     if (!v->tc_cast && !aligned16(I)) return VAICU_ERR_UNSUPPORTED;
     if (v->tc_cast && (reinterpret_cast<uintptr_t>(I) & 3u)) return VAICU_ERR_ALIGNMENT;
     const bool in_cluster = v->tcp.cfold != 0u;       // the K splits fold inside clusters: no partial sums, no fold launch

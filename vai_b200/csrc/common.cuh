@@ -180,7 +180,7 @@ cudaError_t launch_gemv_stream(const LinearArgs& a, const GemvConfig& cfg, uint3
 constexpr uint32_t kSkinnyStreamRows = 8;
 // Whether 5 to 8 rows over [N, K] 16-bit weights are faster there than on the tcgen05 kernel.
 bool skinny_stream_fits(uint32_t N, uint32_t K, bool gate, int sm_count);
-// 1 <= M <= kSkinnyStreamRows, 16-bit weights, K % 8 == 0, I and W 16-byte aligned (skinny_stream.cu)
+// 1 <= M <= kSkinnyStreamRows, 16-bit weights, K % 8 == 0, W and 16-bit I 16-byte aligned (skinny_stream.cu)
 cudaError_t launch_skinny_stream(const LinearArgs& a, int sm_count, uint32_t nseg, const uint32_t* rows, const void* const* w,
                                  void* const* o, cudaStream_t stream);
 

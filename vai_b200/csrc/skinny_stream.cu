@@ -40,12 +40,20 @@ template <> __device__ __forceinline__ void mma16816<__nv_bfloat16>(float* c, ui
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Eight consecutive activations as 16-bit pairs of the weights' type (fp32 ones rounded, as the tcgen05 path's cast does).
-template <typename TW> __device__ __forceinline__ uint4 load_x8(const LinearArgs& a, size_t at)
+// Eight consecutive activations as 16-bit pairs of the weights' type (fp32 ones rounded, as the tcgen05 path's cast does;
+// those may lie at any element, aligned: on 16 bytes).
+template <typename TW> __device__ __forceinline__ uint4 load_x8(const LinearArgs& a, size_t at, bool aligned)
 {
     if (a.i_dtype != VAICU_DTYPE_F32) return *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.I) + at);
-    const float4* s = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.I) + at);
-    const float4 lo = s[0], hi = s[1];
+    const float* s = reinterpret_cast<const float*>(a.I) + at;
+    float4 lo, hi;
+    if (aligned) {
+        lo = reinterpret_cast<const float4*>(s)[0];
+        hi = reinterpret_cast<const float4*>(s)[1];
+    } else {
+        lo = make_float4(s[0], s[1], s[2], s[3]);
+        hi = make_float4(s[4], s[5], s[6], s[7]);
+    }
     uint4 o;
     if constexpr (std::is_same<TW, __half>::value) {
         __half2 h0 = __floats2half2_rn(lo.x, lo.y), h1 = __floats2half2_rn(lo.z, lo.w);
@@ -124,6 +132,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) skinny_stream_kernel(const 
     const EpilogueArgs ep = make_epilogue_args(a);
     uint32_t slot = 0;
     uint4 xb[SC][2];
+    const bool x_aligned = (reinterpret_cast<uintptr_t>(a.I) & 15u) == 0u;
     dependency_wait();
     for (uint32_t b0 = u0; b0 < u1; b0 += kBatchTiles * T) {
         const uint32_t b1 = b0 + kBatchTiles * T < u1 ? b0 + kBatchTiles * T : u1;
@@ -134,7 +143,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) skinny_stream_kernel(const 
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const uint32_t k = (c0 + c) * kChunk + k_lane + h * 32u;
-                        xb[c][h] = (g < M && k < K) ? load_x8<TW>(a, (size_t)g * K + k) : make_uint4(0, 0, 0, 0);
+                        xb[c][h] = (g < M && k < K) ? load_x8<TW>(a, (size_t)g * K + k, x_aligned) : make_uint4(0, 0, 0, 0);
                     }
             }
             uint32_t tile = 0;

@@ -233,9 +233,8 @@ class LinearNode(Node):
         def launch(stream):
             _lib.check(run(plans, n, stream, x, ws, outs, work), "vaicu_linear_run_group")
 
-        rows = first["in0"].num_elements() // first["weight"].shape[1]
-        if first.info.kernel in (KERNEL_GEMV, KERNEL_TC_GEMM) or (rows <= 8 and all(g.info.launches == 1 for g in group)):
-            launch.kernel_launches = 1        # (up to 8 rows on the tensor cores: the streaming form)
+        if need.value == 0:                   # a weight-streaming kernel or the CTA-pair GEMM
+            launch.kernel_launches = 1
         else:
             # GEMM (+ the cast of fp32 activations) (+ the fold, unless the K splits fold inside clusters:
             # then the group needs no room for partial sums)
