@@ -170,8 +170,8 @@ def test_fused_argmax_stores_the_logits_of_a_run(M, kernel, dt, device):
 
 @pytest.mark.parametrize("K,N,gate,streamed", [
     (2048, 8192, False, True), (2048, 148 * 96, False, True), (2048, 148 * 96 + 1, False, False), (1536, 148 * 96 + 1, False, True),
-    (768, 148 * 112 + 1, False, False), (2048, 128256, False, False), (64, 16384, False, False), (2048, 148 * 96, True, True),
-    (2048, 148 * 96 + 2, True, False), (8192, 2048, False, True), (8192, 148 * 16 + 1, False, False), (8192, 148 * 7, False, False),
+    (768, 148 * 112 + 1, False, False), (2048, 128256, False, False), (64, 16384, False, False), (2048, 16384, True, True),
+    (2048, 148 * 112 + 2, True, False), (2056, 148 * 96 + 2, True, False), (8192, 2048, False, True), (8192, 148 * 16 + 1, False, False), (8192, 148 * 7, False, False),
     (8200, 2048, False, False), (12288, 300, False, False)])
 def test_five_to_eight_rows_choice(K, N, gate, streamed, device):
     """Which layers of 5 to 8 rows take the one-launch form: fp32 activations, so the tcgen05 kernel has a cast ahead of it."""

@@ -213,7 +213,8 @@ template <typename TW> cudaError_t launch_skinny_typed(const StreamParams& p, in
 // activations, K 64 to 16384, 16 to 131072 weight rows; us at 8 rows, bf16, here / there:
 //   * every pair of tiles ends in a fold during which the block multiplies nothing, so up to six tiles per block:
 //     2048 x 8192 10.1 / 11.5, 4096 x 8192 (four) as fast, 2048 x 16384 (seven) 16.0 / 13.6, 2048 x 128256 103 / 79; seven while
-//     a tile is short: 1024 x 16384 7.8 / 9.0, but 64 x 16384 (all fold) 5.5 / 3.9;
+//     a tile is short: 1024 x 16384 7.8 / 9.0, but 64 x 16384 (all fold) 5.5 / 3.9; and gated up to K = 2048: 2048 x 16384
+//     15.7 / 15.1, but a recorded Llama-3.2-1B step with fp32 activations 708 / 749 (three launches more per block);
 //   * beyond K = 4096 the activations leave the registers between two pairs of tiles: only layers of one tile per block, at least half
 //     full: 8192 x 2048 9.5 / 10.9, 8192 x 2560 (two) 16.1 / 12.1, 8192 x 300 7.2 / 6.3, 12288 x 300 13.2 / 7.3.
 // The choice is 0.6 % off the better of the two on average, 15 % at most.
@@ -221,7 +222,7 @@ bool skinny_stream_fits(uint32_t N, uint32_t K, bool gate, int sm_count)
 {
     const uint32_t H = gate ? N / 2u : N, tile = gate ? kTileRows / 2u : kTileRows;
     const uint32_t cols = (H + (uint32_t)sm_count - 1u) / (uint32_t)sm_count, tiles = (cols + tile - 1u) / tile;
-    if (K <= 4096u) return tiles <= (K >= 256u && K <= 1536u ? 7u : 6u);
+    if (K <= 4096u) return tiles <= (K >= 256u && K <= (gate ? 2048u : 1536u) ? 7u : 6u);
     return K <= 8192u && tiles == 1u && cols * 2u >= tile;
 }
 
