@@ -498,8 +498,11 @@ cudaError_t launch_one(const GemvParams& p, const GemvConfig& cfg, cudaStream_t 
     auto kern = gemv_kernel<TW, M, R, U>;
     static SmemOptIn optin;
     // One row: the loads in flight land in L1, and behind the streaming form (most of the SM as shared memory) there is room for
-    // 28 KB of them instead of 128: the lm_head of a recorded Llama-3.2-1B step lost 55 us that way.
-    if (cudaError_t e = optin.ensure(kern, 100 * 1024, M == 1 ? (int)cudaSharedmemCarveoutMaxL1 : -1); e != cudaSuccess) return e;
+    // 28 KB of them instead of 128: the lm_head of a recorded Llama-3.2-1B step lost 55 us that way.  The blocks themselves take
+    // 3.3 KB each: two (four k-steps in flight) fit the smallest share, 8 KB; three need the next, 16 of 228 KB
+    // (1 x 2048 x 1536: 5.0 us with two resident blocks, 3.0 with three).
+    const int share = M != 1 ? -1 : (U == 4 ? (int)cudaSharedmemCarveoutMaxL1 : 8);
+    if (cudaError_t e = optin.ensure(kern, 100 * 1024, share); e != cudaSuccess) return e;
     // Programmatic stream serialization: this launch may begin while the kernel ahead
     // of it in the stream drains; gemv_kernel itself waits (dependency_wait) before it
     // reads anything that kernel produced.
