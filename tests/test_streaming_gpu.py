@@ -190,3 +190,25 @@ def test_five_to_eight_rows_on_both_sides_of_the_choice(M, K, N, device):
     x, w, b, r = _draw(M, K, N)
     got, want, _ = run_linear(x, w, b, r, w_dtype="bf16")
     assert_close(got, want, (1e-4, 1e-5), f"{M}x{K}x{N}")
+
+
+@pytest.mark.parametrize("K,N,w,streamed", [
+    (200, 768, "bf16", True), (200, 9000, "bf16", False), (568, 9000, "bf16", False), (576, 9000, "bf16", True), (768, 90000, "bf16", True), (768, 93000, "bf16", False), (8192, 8192, "bf16", True),
+    (8200, 9000, "bf16", False), (400, 32768, "f32", True), (280, 32768, "f32", False), (16392, 3000, "bf16", False)])
+def test_one_row_choice(K, N, w, streamed, device):
+    """Which layers of one row stream: the block count shows in the workspace of the fused Argmax (8 bytes per block)."""
+    d = _lib.LinearDesc(M=1, N=N, K=K, i_dtype=int(Dtype.F32), w_dtype=int(Dtype.BF16 if w == "bf16" else Dtype.F32), o_dtype=int(Dtype.F32),
+                        b_dtype=int(Dtype.NONE), scalar_scale=1.0)
+    plan, need, sms = ctypes.c_void_p(), ctypes.c_size_t(), ctypes.c_int()
+    _lib.check(device.lib.vaicu_device_sm_count(device.handle, ctypes.byref(sms)), "sm_count")
+    _lib.check(device.lib.vaicu_linear_plan_create(device.handle, ctypes.byref(d), ctypes.byref(plan)), "plan")
+    _lib.check(device.lib.vaicu_linear_argmax_workspace_bytes(plan, ctypes.byref(need)), "workspace")
+    assert (need.value == 256 + (sms.value * 8 + 255) // 256 * 256) == streamed
+    device.lib.vaicu_linear_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("K,N,w", [(200, 148 * 16, "bf16"), (200, 148 * 16 + 1, "bf16"), (280, 32768, "f32"), (8200, 9000, "bf16")])
+def test_one_row_on_both_sides_of_the_choice(K, N, w, device):
+    x, wt, b, r = _draw(1, K, N)
+    got, want, _ = run_linear(x, wt, b, r, w_dtype=w)
+    assert_close(got, want, (1e-4, 1e-5), f"1x{K}x{N}")

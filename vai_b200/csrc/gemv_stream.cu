@@ -251,15 +251,22 @@ cudaError_t launch_stream_typed(const StreamParams& p, int xv, int grid, cudaStr
 
 // Geometry of the streaming form; false where it does not apply: more than one row (with 2 to 4 the folds of every row's
 // sums take longer than the loads: 2560 x 20480 bf16, 31 / 51 / 61 us against the register form's 21 / 25 / 30), K too long
-// for the registers that hold the activations, or a layer so large that the hand-over no longer counts (the register
-// form keeps 128 KB per SM on their way instead of 96: a 3072 x 128256 head takes 112 us there and 136 us here).
+// for the registers that hold the activations, and where the register form is the better one (here / there, us, in recorded
+// chains of one layer, 700 layers, K 64 to 16384):
+//   * above 140 MB, where the hand-over no longer counts and the register form keeps 128 KB per SM on their way instead of 96:
+//     201 MB layers 33.6 / 33.6 (1536 x 65536), 44.1 / 36.8 (5000 x 20000), 148 MB 36.0 / 27.3 (8200 x 9000); still ahead at
+//     134 MB 21.3 / 24.1 (8192 x 8192) and 105 MB 17.5 / 19.8 (2560 x 20480);
+//   * where K fills less than three quarters of the vectors that the lanes load, and a block has more than two rounds of
+//     rows: 200 x 32768 10.5 / 6.8, 400 x 8192 4.1 / 3.2, 552 x 9000 4.3 / 3.9, but 200 x 768 (one round) 1.9 / 2.0.
+// Of the layers that stay, most gain 5 to 30 %; the losses are up to 16 % at 8 to 13 MB, about one FIFO per SM (2048 x 2560 4.0 / 3.5,
+// while 2560 x 2048 takes 3.5 / 4.0).
 // The warps per row: the fewest rounds of rows per block, weighed by the vectors of a round and 1.5 for its fold.
 bool choose_gemv_stream(const LinearArgs& a, int sm_count, GemvStream* out)
 {
     GemvStream c{};
     const uint32_t esz = dtype_size(a.w_dtype), vec = 16u / esz;
     const uint32_t H = a.gate_fuse ? a.N / 2u : a.N;
-    if (a.M != 1u || a.K % vec || H == 0u || (uint64_t)a.N * a.K * esz > 200000000ull) return false;
+    if (a.M != 1u || a.K % vec || H == 0u || (uint64_t)a.N * a.K * esz > 140000000ull) return false;
     const uint32_t nvec = a.K / vec, units = (H + (uint32_t)sm_count - 1u) / (uint32_t)sm_count;
     uint32_t ks = 0u;
     double best = 1e30;
@@ -273,8 +280,9 @@ bool choose_gemv_stream(const LinearArgs& a, int sm_count, GemvStream* out)
     }
     if (!ks) return false;
     c.ks = ks;
+    const uint32_t rg = kStreamWarps / ks, slots = 32u * ks * (uint32_t)c.xv;
+    if (nvec * 4u < slots * 3u && units > 2u * rg) return false;
     // whole rounds of the warps' row groups between two folds
-    const uint32_t rg = kStreamWarps / ks;
     c.batch = kPartFloats / ((a.gate_fuse ? 2u : 1u) * ks) / rg * rg;
     c.grid = (int)(H < (uint32_t)sm_count ? H : (uint32_t)sm_count);
     *out = c;
