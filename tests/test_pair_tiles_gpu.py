@@ -1,12 +1,14 @@
 """The CTA-pair kernel at every width its cost model picks from, whole and split along K: ragged rows and columns, K tails,
 fewer k-blocks than stages, finished tiles stored through shared memory or directly, partial sums as whole or single
 elements (N % 4 != 0), residuals one chunk ahead."""
+import ctypes
+
 import numpy as np
 import pytest
 from gpu_util import out_tol, run_linear
 from linear_check import assert_close
 
-from vai_b200 import nodes
+from vai_b200 import Dtype, _lib, nodes
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +48,23 @@ def test_chosen_tiles(M, K, N, device):
     got, want, node = run_linear(x, w, b, r, w_dtype="bf16")
     assert node.info.kernel == (nodes.KERNEL_TC_GEMM if M > 128 else nodes.KERNEL_TC_SKINNY)
     assert_close(got, want, (2e-4, 5e-5), f"{M}x{K}x{N}")
+
+
+@pytest.mark.parametrize("M,K,N,gate,widest", [(40000, 768, 64, False, 64), (40000, 768, 100, False, 128), (20000, 2048, 300, False, 192),
+                                               (40000, 768, 768, False, 256), (8192, 768, 2048, False, 256), (40000, 768, 2 * 40, True, 64)])
+def test_tall_layers_do_not_compute_padding(M, K, N, gate, widest, device):
+    """Many rounds of tiles, few columns: the widest tile only where the output fills it."""
+    d = _lib.LinearDesc(M=M, N=N, K=K, i_dtype=int(Dtype.BF16), w_dtype=int(Dtype.BF16), o_dtype=int(Dtype.BF16), b_dtype=int(Dtype.NONE),
+                        scalar_scale=1.0, gate_fuse=int(gate))
+    plan, info = ctypes.c_void_p(), _lib.LinearInfo()
+    _lib.check(device.lib.vaicu_linear_plan_create(device.handle, ctypes.byref(d), ctypes.byref(plan)), "plan")
+    _lib.check(device.lib.vaicu_linear_plan_info(plan, ctypes.byref(info)), "info")
+    assert info.tile_n == widest
+    device.lib.vaicu_linear_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("M,N", [(9480 * 2, 300), (40000, 64)])
+def test_tall_layers(M, N, device):
+    x, w, b, _ = _draw(M, 72, N)
+    got, want, _ = run_linear(x, w, b, i_dtype="bf16", w_dtype="bf16", o_dtype="bf16")
+    assert_close(got, want, out_tol("bf16", 2e-4, 5e-5), f"{M}x72x{N}")

@@ -249,7 +249,9 @@ bool tc_eligible(const vaicu_linear_desc& d)
 // A k-block takes 0.19 us at 64 columns and hardly more up to 128 (issue and L2 set the pace), 0.255 at 192, 0.32 at 256
 // (the MMAs do); a last round of few tiles runs as column strips.  Measured over 19 layers x 160-2000 rows, all
 // five widths and up to 8 splits: the choice is 0.5 % off the best on average, 14 % at most (whole-wave rule before: 5 %).
-// From two full rounds of 256-column tiles on those are taken: wider tiles read the operands less often.
+// From two full rounds of 256-column tiles on those are taken, as long as the output fills seven eighths of their columns: wider
+// tiles read the operands less often, but a tall layer of few columns would compute mostly padding (40000 x 768 x 64: 23.6 us in
+// tiles of 256 columns, 20.9 in 64).
 uint32_t choose_pair_tile(const vaicu_linear_desc& d, uint32_t units, uint32_t* splits)
 {
     const bool gate = d.gate_fuse != 0;
@@ -257,7 +259,8 @@ uint32_t choose_pair_tile(const vaicu_linear_desc& d, uint32_t units, uint32_t* 
     const uint32_t cand[5] = {64u, 96u, 128u, 192u, 256u};
     const double per_kb[5] = {0.19, 0.225, 0.22, 0.255, 0.32};
     *splits = 1u;
-    if (tiles_m * ceil_div(H, gate ? 128u : 256u) >= 2u * units) return 256u;
+    const uint32_t widest = gate ? 128u : 256u, across = ceil_div(H, widest);
+    if (tiles_m * across >= 2u * units && H * 8u >= across * widest * 7u) return 256u;
     uint32_t best_bn = 256u;
     double best = 1e30;
     for (int i = 0; i < 5; ++i) {
