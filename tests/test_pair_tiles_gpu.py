@@ -68,3 +68,13 @@ def test_tall_layers(M, N, device):
     x, w, b, _ = _draw(M, 72, N)
     got, want, _ = run_linear(x, w, b, i_dtype="bf16", w_dtype="bf16", o_dtype="bf16")
     assert_close(got, want, out_tol("bf16", 2e-4, 5e-5), f"{M}x72x{N}")
+
+
+@pytest.mark.parametrize("bn", [64, 128, 192, 256])
+@pytest.mark.parametrize("M,N,gate", [(129, 333, False), (300, 1001, False), (520, 2 * 333, True), (257, 129, False)])
+def test_rows_of_odd_width_in_fp32(bn, M, N, gate, device):
+    """Output rows that begin at any fp32 element go through shared memory too, a store instruction per row."""
+    x, w, b, r = _draw(M, 200, N)
+    got, want, node = run_linear(x, w, b, None if gate else r, i_dtype="bf16", w_dtype="bf16", epilogue="GELU" if gate else "SILU", gate_fuse=gate,
+                                 kernel=nodes.KERNEL_TC_GEMM, tuning=dict(tc_pair=1, tc_bn=bn, tc_splits=1))
+    assert_close(got, want, (2e-4, 5e-5), f"{M}x200x{N} bn={bn}")
