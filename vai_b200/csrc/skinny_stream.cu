@@ -41,13 +41,13 @@ template <> __device__ __forceinline__ void mma16816<__nv_bfloat16>(float* c, ui
 }
 
 // Eight consecutive activations as 16-bit pairs of the weights' type (fp32 ones rounded, as the tcgen05 path's cast does;
-// those may lie at any element, aligned: on 16 bytes).
-template <typename TW> __device__ __forceinline__ uint4 load_x8(const LinearArgs& a, size_t at, bool aligned)
+// without XA those may begin at any element).
+template <typename TW, bool XA> __device__ __forceinline__ uint4 load_x8(const LinearArgs& a, size_t at)
 {
     if (a.i_dtype != VAICU_DTYPE_F32) return *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.I) + at);
     const float* s = reinterpret_cast<const float*>(a.I) + at;
     float4 lo, hi;
-    if (aligned) {
+    if constexpr (XA) {
         lo = reinterpret_cast<const float4*>(s)[0];
         hi = reinterpret_cast<const float4*>(s)[1];
     } else {
@@ -71,7 +71,8 @@ template <typename TW> __device__ __forceinline__ uint4 load_x8(const LinearArgs
 
 // SC: chunks of K whose activations are held in registers at a time.  Order of work: batches of tiles; per batch, spans
 // of SC chunks; per span the batch's tiles; per tile the span's chunks.
-template <typename TW, int SC>
+// XA: the activations are 16-byte aligned.
+template <typename TW, int SC, bool XA>
 __global__ void __launch_bounds__(kStreamThreads, 2) skinny_stream_kernel(const StreamParams p)
 {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -132,7 +133,6 @@ __global__ void __launch_bounds__(kStreamThreads, 2) skinny_stream_kernel(const 
     const EpilogueArgs ep = make_epilogue_args(a);
     uint32_t slot = 0;
     uint4 xb[SC][2];
-    const bool x_aligned = (reinterpret_cast<uintptr_t>(a.I) & 15u) == 0u;
     dependency_wait();
     for (uint32_t b0 = u0; b0 < u1; b0 += kBatchTiles * T) {
         const uint32_t b1 = b0 + kBatchTiles * T < u1 ? b0 + kBatchTiles * T : u1;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kStreamThreads, 2) skinny_stream_kernel(const 
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const uint32_t k = (c0 + c) * kChunk + k_lane + h * 32u;
-                        xb[c][h] = (g < M && k < K) ? load_x8<TW>(a, (size_t)g * K + k, x_aligned) : make_uint4(0, 0, 0, 0);
+                        xb[c][h] = (g < M && k < K) ? load_x8<TW, XA>(a, (size_t)g * K + k) : make_uint4(0, 0, 0, 0);
                     }
             }
             uint32_t tile = 0;
@@ -195,16 +195,18 @@ __global__ void __launch_bounds__(kStreamThreads, 2) skinny_stream_kernel(const 
     }
 }
 
-template <typename TW, int SC> cudaError_t launch_skinny_form(const StreamParams& p, int grid, cudaStream_t stream)
+template <typename TW, int SC, bool XA> cudaError_t launch_skinny_form(const StreamParams& p, int grid, cudaStream_t stream)
 {
-    auto kern = skinny_stream_kernel<TW, SC>;
+    auto kern = skinny_stream_kernel<TW, SC, XA>;
     static SmemOptIn optin;
     if (cudaError_t e = optin.ensure(kern, (int)kSkinnySmem, cudaSharedmemCarveoutMaxShared); e != cudaSuccess) return e;
     return launch_pdl(kern, dim3((unsigned)grid), dim3(kStreamThreads), kSkinnySmem, stream, p);
 }
 template <typename TW> cudaError_t launch_skinny_typed(const StreamParams& p, int grid, cudaStream_t stream)
 {
-    return p.a.K <= 4u * kChunk ? launch_skinny_form<TW, 4>(p, grid, stream) : launch_skinny_form<TW, 8>(p, grid, stream);
+    if ((reinterpret_cast<uintptr_t>(p.a.I) & 15u) == 0u)
+        return p.a.K <= 4u * kChunk ? launch_skinny_form<TW, 4, true>(p, grid, stream) : launch_skinny_form<TW, 8, true>(p, grid, stream);
+    return p.a.K <= 4u * kChunk ? launch_skinny_form<TW, 4, false>(p, grid, stream) : launch_skinny_form<TW, 8, false>(p, grid, stream);
 }
 
 }  // namespace
