@@ -391,10 +391,8 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
     auto size_ring = [&](uint32_t extra) {
         uint32_t stages = (uint32_t)((kTcMaxSmem - 2048u - extra) / stage_bytes);
         if (stages > 8u) stages = 8u;
-        // A CTA of the swapped kernel that streams only a few k-blocks (a K split of a small layer) gets a
-        // ring of four stages: two such CTAs then fit on an SM, so the next launch's CTAs set up and request
-        // their weights while this launch's finish (q / o of a 4B-class model at batch 64: 8.3 -> 7.7 us and
-        // 8.8 -> 8.1 us; layers with long K ranges lose with the short ring and keep the deep one).
+        // A CTA of the swapped kernel that streams only a few k-blocks (a K split of a small layer) needs no deep ring; the full
+        // one is 0.2 % slower over 468 layers at 9 to 128 rows (6 % at 128 x 8192 x 1024, 3 % faster at 64 x 2560 x 2048).
         if (swap && t.splits > 1u && t.kb_per_split <= 10u && stages > 4u) stages = 4u;
         if (pl->tune.tc_stages && pl->tune.tc_stages < stages) stages = pl->tune.tc_stages;
         t.stages = stages;
