@@ -303,8 +303,10 @@ VAICU_API int vaicu_linear_run_group(vaicu_linear_plan* const* plans, int count,
  * vaicu_ipc_open} the epilogue of the tensor-core kernel performs the all-gather itself
  * with plain stores over NVLink, tile by tile, instead of a collective after the kernel;
  * the ranks still need one synchronisation before anyone reads the gathered output.
- * Tensor-core plans without split-K and without residual only (VAICU_ERR_UNSUPPORTED
- * otherwise); destinations 16-byte aligned.  No counterpart in the single-device reference. */
+ * Tensor-core plans without residual whose K stays whole only (VAICU_ERR_UNSUPPORTED otherwise):
+ * a K split that the library chose for speed is left out here, one that the caller asked for
+ * (split_size, tc_splits) is not, nor one that a layer of less than half a tile per SM needs;
+ * destinations 16-byte aligned.  No counterpart in the single-device reference. */
 VAICU_API int vaicu_linear_run_scatter(vaicu_linear_plan* plan, vaicu_stream_t stream, const void* I, const void* W,
                                        const void* bias, void* const* dsts, int n_dst, uint32_t ldo, uint32_t col0,
                                        void* workspace);
@@ -313,8 +315,8 @@ VAICU_API int vaicu_linear_run_scatter(vaicu_linear_plan* plan, vaicu_stream_t s
  * [M_total, N] tensor, ranks that each run the Linear on their own rows of the activations assemble the
  * full result everywhere inside their GEMM epilogues (an all-gather along rows, as a sequence-parallel
  * block needs in front of its column-split MLP).  Bias, epilogue, residual and scale as in
- * vaicu_linear_run (they index the plan's own [M, N]).  Tensor-core plans without split-K only;
- * destinations 16-byte aligned; the ranks synchronise (vaicu_peer_barrier_run) before anyone reads.
+ * vaicu_linear_run (they index the plan's own [M, N]).  Plans as for
+ * vaicu_linear_run_scatter, residual allowed; destinations 16-byte aligned; the ranks synchronise (vaicu_peer_barrier_run) before anyone reads.
  * No counterpart in the single-device reference. */
 VAICU_API int vaicu_linear_run_broadcast(vaicu_linear_plan* plan, vaicu_stream_t stream, const void* I, const void* W,
                                          const void* bias, const void* residual, void* const* dsts, int n_dst,

@@ -142,6 +142,8 @@ struct vaicu_linear_plan {
     int last_kernel, last_vectorized;
     // this plan as the first member of a group on the tensor-core kernel (vaicu_linear_run_group)
     struct GroupState* group;
+    // the same Linear in whole waves of tiles, for runs with several destinations (whole_plan)
+    vaicu_linear_plan* whole;
 };
 
 // Two or three plans on the swapped tensor-core kernel run as one Linear over their weights' rows
@@ -283,10 +285,32 @@ uint32_t choose_pair_tile(const vaicu_linear_desc& d, uint32_t units, uint32_t* 
     return best_bn;
 }
 
+// Columns per tile by whole waves of 256, 128 or 64 columns over `units`; f128, f64: what a narrower tile costs, which
+// re-reads the activations more often and issues shorter MMAs.
+uint32_t choose_wave_tile(const vaicu_linear_desc& d, uint32_t tile_rows, uint32_t units, double f128, double f64)
+{
+    const bool gate = d.gate_fuse != 0;
+    const uint32_t H = gate ? d.N / 2u : d.N, cand[3] = {256u, 128u, 64u};
+    uint32_t bn = 256u;
+    double best = -1.0;
+    for (uint32_t c : cand) {
+        const uint32_t out_cols = gate ? c / 2u : c;
+        const uint32_t tiles = ceil_div(d.M, tile_rows) * ceil_div(H, out_cols);
+        const uint32_t waves = ceil_div(tiles, units);
+        double eff = (double)tiles / ((double)waves * units);
+        eff *= (c == 256u) ? 1.0 : (c == 128u ? f128 : f64);
+        // a tile wider than the whole output is wasted work
+        if (out_cols > (uint32_t)align_up(H, 16u) && c != 64u) eff *= (double)H / out_cols;
+        if (eff > best) { best = eff; bn = c; }
+    }
+    return bn;
+}
+
 // Tile / split choice of the tensor-core kernel (the role selectLinearTile plays
 // in the reference, vAi linear.h:2101-2119): fill the SMs with whole waves of
 // the widest tile, and split K only when the tile grid cannot occupy them.
-void plan_tc(vaicu_linear_plan* pl, bool swap)
+// in_waves: no split that only makes the layer faster, K stays whole unless the tiles leave half the SMs idle.
+void plan_tc(vaicu_linear_plan* pl, bool swap, bool in_waves)
 {
     const vaicu_linear_desc& d = pl->d;
     const uint32_t sms = (uint32_t)pl->dev->sm_count;
@@ -315,7 +339,7 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
         uint64_t best_cost = ~0ull;
         // At least 64 rows without a gate: below, a layer of 2560-4700 rows would just fit the SMs unsplit with a quarter of
         // the loads in flight (K = 8192, N = 3072 at 24 rows of activations: 38 us in 40-row tiles, 14 us split).
-        for (uint32_t rows = 128u; rows >= (gate ? 32u : 64u) && !d.split_size; rows -= 8u) {
+        for (uint32_t rows = 128u; rows >= (gate || in_waves ? 32u : 64u) && !d.split_size; rows -= 8u) {
             if (boxes * rows < bn) break;
             const uint32_t tiles = ceil_div(H, rows) * t.tiles_b;
             if (tiles * 2u <= sms) continue;
@@ -332,23 +356,9 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
         if (pl->tune.tc_pair >= 0) pair = pl->tune.tc_pair != 0;
         // output columns per tile: bn (bn / 2 with gate)
         bn = 256u;
-        if (pair) {
-            bn = choose_pair_tile(d, sms / 2u, &pair_splits);
-        } else {
-            const uint32_t cand[3] = {256u, 128u, 64u};
-            double best = -1.0;
-            for (uint32_t c : cand) {
-                const uint32_t out_cols = gate ? c / 2u : c;
-                const uint32_t tiles = ceil_div(d.M, 128u) * ceil_div(H, out_cols);
-                const uint32_t waves = ceil_div(tiles, sms);
-                double eff = (double)tiles / ((double)waves * sms);
-                // narrower tiles re-read the activations more often and issue shorter MMAs
-                eff *= (c == 256u) ? 1.0 : (c == 128u ? 0.88 : 0.70);
-                // a tile wider than the whole output is wasted work
-                if (out_cols > (uint32_t)align_up(H, 16u) && c != 64u) eff *= (double)H / out_cols;
-                if (eff > best) { best = eff; bn = c; }
-            }
-        }
+        if (!pair) bn = choose_wave_tile(d, 128u, sms, 0.88, 0.70);
+        else if (in_waves) bn = choose_wave_tile(d, 256u, sms / 2u, 0.70, 0.45);
+        else bn = choose_pair_tile(d, sms / 2u, &pair_splits);
         if (pl->tune.tc_bn) bn = pl->tune.tc_bn;   // validated when the plan was created
         // Single-CTA alternative for 256-row tiles: two A boxes per stage and two MMAs per
         // k-step; needs all 512 TMEM columns at bn = 256 (no epilogue overlap).
@@ -368,7 +378,7 @@ void plan_tc(vaicu_linear_plan* pl, bool swap)
     uint32_t kb_per_split = t.kblocks;
     if (d.split_size) {
         kb_per_split = ceil_div(d.split_size, 64u);
-    } else if (t.pair && !pl->tune.tc_bn) {
+    } else if (t.pair && !pl->tune.tc_bn && !in_waves) {
         kb_per_split = ceil_div(t.kblocks, pair_splits);
     } else if (t.num_tiles * 2u <= units && t.kblocks >= 8u) {
         uint32_t want = units / t.num_tiles;
@@ -530,7 +540,7 @@ bool tunes_tc(const vaicu_linear_tuning& t)
     return t.tc_pair >= 0 || t.tc_wide >= 0 || t.tc_bn || t.tc_splits || t.tc_fold || t.tc_stages || t.tc_tile_rows || t.tc_tail_strips;
 }
 
-int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_linear_tuning& tuning, vaicu_linear_plan** out)
+int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_linear_tuning& tuning, vaicu_linear_plan** out, bool in_waves = false)
 {
     if (!dev || !out) return VAICU_ERR_INVALID_VALUE;
     int rc = validate_desc(desc);
@@ -545,6 +555,7 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
     pl->tune = tuning;
     pl->tile_done = nullptr;
     pl->group = nullptr;
+    pl->whole = nullptr;
     if (!pl->d.has_bias) { pl->d.bias_elems = 0; pl->d.b_dtype = VAICU_DTYPE_NONE; }
     if (!pl->d.has_residual) pl->d.residual_elems = 0;
     // a [N] bias under M == 1 "covers O" (elems 0); name it per-row so every kernel takes the cheap index
@@ -580,7 +591,7 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
     case VAICU_KERNEL_TC_SKINNY:
         if (!tc_eligible(d) || (kernel == VAICU_KERNEL_TC_SKINNY && d.M > 256u)) { delete pl; return VAICU_ERR_UNSUPPORTED; }
         pl->tc = true;
-        plan_tc(pl, kernel == VAICU_KERNEL_TC_SKINNY);
+        plan_tc(pl, kernel == VAICU_KERNEL_TC_SKINNY, in_waves);
         pl->workspace_bytes = pl->ws_cast_bytes + pl->ws_partial_bytes;
         // unaligned operands fall back to the FMA tile kernel at run time
         if (pl->fma_ws_bytes > pl->workspace_bytes) pl->workspace_bytes = pl->fma_ws_bytes;
@@ -614,6 +625,25 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
     pl->map_a_next = pl->map_b_next = 0u;
     *out = pl;
     return VAICU_OK;
+}
+
+// The plan for a run with several destinations, whose epilogue must see finished sums: this one, or, where the library split
+// its K by its own choice, the same Linear in whole waves of tiles, made on first use and kept.
+int whole_plan(vaicu_linear_plan* pl, vaicu_linear_plan** out)
+{
+    if (!pl->tc) return VAICU_ERR_UNSUPPORTED;
+    *out = pl;
+    if (pl->tcp.splits == 1u) return VAICU_OK;
+    if (pl->d.split_size || pl->tune.tc_splits) return VAICU_ERR_UNSUPPORTED;
+    if (!pl->whole) {
+        vaicu_linear_tuning tune = pl->tune;
+        tune.kernel = pl->kernel;
+        tune.tc_fold = 0;
+        const int rc = build_plan(pl->dev, &pl->d, tune, &pl->whole, true);
+        if (rc != VAICU_OK) return rc;
+    }
+    *out = pl->whole;
+    return pl->whole->tcp.splits == 1u ? VAICU_OK : VAICU_ERR_UNSUPPORTED;
 }
 
 int run_fma(vaicu_linear_plan* pl, const LinearArgs& a, void* workspace, cudaStream_t s)
@@ -900,6 +930,7 @@ int vaicu_linear_plan_destroy(vaicu_linear_plan* plan)
         vaicu_linear_plan_destroy(plan->group->virt);
         delete plan->group;
     }
+    if (plan->whole) vaicu_linear_plan_destroy(plan->whole);
     delete plan;
     return VAICU_OK;
 }
@@ -945,6 +976,15 @@ struct OutputSpec {
 };
 int run_impl(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const void* W, const void* bias,
              const void* residual, void* O, void* workspace, const OutputSpec* spec);
+// A run on whole_plan(pl), reported by vaicu_linear_plan_last_run as one on pl.
+int run_whole(vaicu_linear_plan* pl, vaicu_linear_plan* whole, vaicu_stream_t stream, const void* I, const void* W, const void* bias,
+              const void* residual, void* O, void* workspace, const OutputSpec& spec)
+{
+    const int rc = run_impl(whole, stream, I, W, bias, residual, O, workspace, &spec);
+    pl->last_kernel = whole->last_kernel;
+    pl->last_vectorized = whole->last_vectorized;
+    return rc;
+}
 }  // namespace
 
 int vaicu_linear_run(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const void* W, const void* bias,
@@ -959,9 +999,10 @@ int vaicu_linear_run_reduce_scatter(vaicu_linear_plan* pl, vaicu_stream_t stream
     if (!pl || !dsts || n_dst < 1 || n_dst > 8 || slot < 0 || slot >= n_dst) return VAICU_ERR_INVALID_VALUE;
     const vaicu_linear_desc& d = pl->d;
     // partial sums only: anything after the dot product belongs to the fold that follows the exchange
-    if (!pl->tc || pl->tcp.splits > 1u || d.has_residual || d.has_bias || d.gate_fuse || d.epilogue != VAICU_EPILOGUE_NONE ||
-        d.scalar_scale != 1.0f)
+    if (d.has_residual || d.has_bias || d.gate_fuse || d.epilogue != VAICU_EPILOGUE_NONE || d.scalar_scale != 1.0f)
         return VAICU_ERR_UNSUPPORTED;
+    vaicu_linear_plan* whole = nullptr;
+    if (const int rc = whole_plan(pl, &whole); rc != VAICU_OK) return rc;
     if (d.M % (uint32_t)n_dst) return VAICU_ERR_INVALID_VALUE;
     OutputSpec spec{};
     spec.n_dst = (uint32_t)n_dst;
@@ -974,7 +1015,7 @@ int vaicu_linear_run_reduce_scatter(vaicu_linear_plan* pl, vaicu_stream_t stream
         if (reinterpret_cast<uintptr_t>(dsts[i]) & 15u) return VAICU_ERR_ALIGNMENT;
         spec.dst[i] = dsts[i];
     }
-    return run_impl(pl, stream, I, W, nullptr, nullptr, dsts[0], workspace, &spec);
+    return run_whole(pl, whole, stream, I, W, nullptr, nullptr, dsts[0], workspace, spec);
 }
 
 int vaicu_partial_fold_run(vaicu_device* dev, vaicu_stream_t stream, const void* parts, uint32_t n_parts, uint32_t rows, uint32_t N,
@@ -1067,7 +1108,9 @@ int vaicu_linear_run_scatter(vaicu_linear_plan* pl, vaicu_stream_t stream, const
     const uint32_t width = d.gate_fuse ? d.N / 2u : d.N;
     if (ldo < width || col0 > ldo - width) return VAICU_ERR_INVALID_VALUE;
     // only the tensor-core kernels write strided slabs, and only without a split-K fold or a residual
-    if (!pl->tc || pl->tcp.splits > 1u || d.has_residual) return VAICU_ERR_UNSUPPORTED;
+    if (d.has_residual) return VAICU_ERR_UNSUPPORTED;
+    vaicu_linear_plan* whole = nullptr;
+    if (const int rc = whole_plan(pl, &whole); rc != VAICU_OK) return rc;
     OutputSpec spec{};
     spec.n_dst = (uint32_t)n_dst;
     spec.ldo = ldo;
@@ -1077,7 +1120,7 @@ int vaicu_linear_run_scatter(vaicu_linear_plan* pl, vaicu_stream_t stream, const
         if (reinterpret_cast<uintptr_t>(dsts[i]) & 15u) return VAICU_ERR_ALIGNMENT;
         spec.dst[i] = dsts[i];
     }
-    return run_impl(pl, stream, I, W, bias, nullptr, dsts[0], workspace, &spec);
+    return run_whole(pl, whole, stream, I, W, bias, nullptr, dsts[0], workspace, spec);
 }
 
 int vaicu_linear_run_broadcast(vaicu_linear_plan* pl, vaicu_stream_t stream, const void* I, const void* W, const void* bias,
@@ -1086,7 +1129,8 @@ int vaicu_linear_run_broadcast(vaicu_linear_plan* pl, vaicu_stream_t stream, con
     if (!pl || !dsts || n_dst < 1 || n_dst > 8) return VAICU_ERR_INVALID_VALUE;
     const vaicu_linear_desc& d = pl->d;
     // the tensor-core kernels' epilogues store to several destinations; a split-K fold does not
-    if (!pl->tc || pl->tcp.splits > 1u) return VAICU_ERR_UNSUPPORTED;
+    vaicu_linear_plan* whole = nullptr;
+    if (const int rc = whole_plan(pl, &whole); rc != VAICU_OK) return rc;
     OutputSpec spec{};
     spec.n_dst = (uint32_t)n_dst;
     spec.ldo = d.gate_fuse ? d.N / 2u : d.N;      // dense destinations: bias and residual index them like O
@@ -1096,7 +1140,7 @@ int vaicu_linear_run_broadcast(vaicu_linear_plan* pl, vaicu_stream_t stream, con
         if (reinterpret_cast<uintptr_t>(dsts[i]) & 15u) return VAICU_ERR_ALIGNMENT;
         spec.dst[i] = dsts[i];
     }
-    return run_impl(pl, stream, I, W, bias, residual, dsts[0], workspace, &spec);
+    return run_whole(pl, whole, stream, I, W, bias, residual, dsts[0], workspace, spec);
 }
 
 namespace {
