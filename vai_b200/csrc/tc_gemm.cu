@@ -604,13 +604,8 @@ __device__ __forceinline__ void tc_trace(uint32_t slot)
 // GATE: fused Linear + GatedMul.  Non-swap: the B stage holds bn/2 gate rows then
 //       bn/2 value rows; swap: the A stage holds 128 gate rows then 128 value rows
 //       and two MMAs per k-step fill two accumulators.
-//
-// Registers: at 159 a thread the swapped kernel's 384 threads left 4096 of an SM's 65536, and the blocks of the fold behind a K
-// split (8192 and 10240) could not move in before it had left.  Bounded to 128 (no spills) they can: 468 layers at 9 to 128 rows,
-// 1.8 % faster on average with 16-bit activations, up to 17 % (64 x 8192 x 512 9.9 -> 8.6 us), 0.9 % with fp32 ones.  The gated form
-// would spill, and rarely has a fold behind it.
 template <bool SWAP, bool GATE>
-__global__ void __launch_bounds__(SWAP && !GATE ? 512 : kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ CUtensorMap tmap_a1, const __grid_constant__ CUtensorMap tmap_a2, const TcParams p)
 {
