@@ -279,8 +279,10 @@ class _LoanPool:
     """The page-locked arrays that one output of a recording is copied into and handed out in.  A large output (a
     prefill's hidden state, one row of logits) reaches the caller in one copy that way; a staging buffer and a fresh
     array cost a second pass over it and a page fault per 4 KB (513 KB of logits: 50 us of a 525 us step).  Two arrays are
-    made with the recording (a caller usually holds the last result while it asks for the next), at most LIMIT
-    exist; a caller that keeps more gets plain copies.  deque's append and pop are atomic, so arrays may die on any
+    made with the recording (a caller usually holds the last result while it asks for the next; the second one takes as
+    long to make as the staging buffer did: 12 ms at 64 MB), at most LIMIT exist: up to 256 MB of page-locked memory for
+    an output of LOAN_MAX_BYTES, per recorded shape, until the recording and the last view of an array are gone.  A caller
+    that keeps more gets plain copies.  deque's append and pop are atomic, so arrays may die on any
     thread, after the recording too."""
     FIRST, LIMIT = 2, 4
 
@@ -405,8 +407,10 @@ class Tensor:
         return bits_to_f32(raw, Dtype.BF16)
 
 
-# Outputs handed out in page-locked arrays.  Below, the copy they save costs less than a command of its own; above, they
-# would pin too much of the host's memory.
+# Outputs handed out in page-locked arrays.  A whole call of a small net, staged and copied / handed out, us: 16 KB 24 / 22,
+# 64 KB 35 / 27, 512 KB 64 / 44, 4 MB 375 / 103, 64 MB 14300 / 1250, 128 MB 28300 / 2500.  Below the range little is saved, and small
+# results are what callers keep many of; above it four arrays would hold more than 256 MB of page-locked memory where
+# the staging buffer holds one.
 LOAN_MIN_BYTES, LOAN_MAX_BYTES = 64 << 10, 64 << 20
 
 # ---- graph: slots, nodes, flows ----------------------------------------------------
@@ -713,6 +717,9 @@ class NeuralNet:
         self._pin_sink = rec.pinned
         try:
             return self._record_into(rec, fed)
+        except BaseException:
+            self._release(rec)
+            raise
         finally:
             self._pin_sink = self._pinned_ptrs
 
@@ -866,20 +873,26 @@ class NeuralNet:
     def _copies_out(self, rec):
         lib = self.device.lib
         for name, t in rec.outputs.items():
-            if name in rec.loans:       # a new destination on every call: _copy_loans
+            if name in rec.loans:       # a new destination on every call: _finish
                 continue
             view, hp = rec.stage_out[name]
             if hp is not None:          # else the kernel wrote the host memory itself
                 _lib.check(lib.vaicu_memcpy_d2h(hp, t.ptr, view.nbytes, self.stream), "vaicu_memcpy_d2h")
 
-    def _copy_loans(self, rec):
-        """Enqueues the copies of the large outputs; {name: host array}, valid once the stream has been waited for."""
+    def _finish(self, rec):
+        """Enqueues the copies of the large outputs and waits for the stream; {name: host array} of those outputs."""
         arrays = {}
-        for name, pool in rec.loans.items():
-            ptr = pool.take()
-            arrays[name] = pool.array(ptr) if ptr is not None else np.empty(pool.shape, dtype=pool.np_dtype)
-            _lib.check(self.device.lib.vaicu_memcpy_d2h(arrays[name].ctypes.data, rec.outputs[name].ptr, pool.nbytes, self.stream),
-                       "vaicu_memcpy_d2h")
+        lib = self.device.lib
+        try:
+            for name, pool in rec.loans.items():
+                ptr = pool.take()
+                arrays[name] = pool.array(ptr) if ptr is not None else np.empty(pool.shape, dtype=pool.np_dtype)
+                _lib.check(lib.vaicu_memcpy_d2h(arrays[name].ctypes.data, rec.outputs[name].ptr, pool.nbytes, self.stream), "vaicu_memcpy_d2h")
+            _lib.check(lib.vaicu_stream_sync(self.stream), "vaicu_stream_sync")
+        except BaseException:
+            if arrays:
+                lib.vaicu_stream_sync(self.stream)       # a copy under way may still write: the arrays go back after it
+            raise
         return arrays
 
     def _play(self, ops):
@@ -942,8 +955,7 @@ class NeuralNet:
             self._copies_in(rec)
             self._play(rec.ops)
             self._copies_out(rec)
-        loaned = self._copy_loans(rec) if rec.loans else {}
-        _lib.check(lib.vaicu_stream_sync(self.stream), "vaicu_stream_sync")
+        loaned = self._finish(rec)
         # the kernels' bounded waits report through a device word: read it on the first
         # replay of a recording and then now and again, not on every step
         if rec.calls % 256 == 0:
@@ -966,23 +978,28 @@ class NeuralNet:
         if lib is not None and self.stream is not None:
             lib.vaicu_stream_sync(self.stream)           # nothing recorded is still running
         for rec in self._recordings.values():
-            for g in (rec.graph, getattr(rec, "graph_io", None)):
-                if g is not None:
-                    lib.vaicu_graph_destroy(g)
-            rec.graph = rec.graph_io = None
-            for pool in rec.loans.values():
-                pool.close()
-            for p in rec.pinned:
-                lib.vaicu_host_free_pinned(p)
-            rec.pinned = []
-            seen_buffers = set()
-            for t in list(rec.input_tensors.values()) + rec.keep:
-                b = t.buffer
-                if isinstance(b, (DeviceBuffer, GuardedBuffer)) and id(b) not in seen_buffers and b.ptr is not None:
-                    seen_buffers.add(id(b))
-                    self.pool.release(b)
-                t.buffer = None
+            self._release(rec)
         self._recordings.clear()
+
+    def _release(self, rec):
+        """Everything made for one recording, also for one that failed half way."""
+        lib = self.device.lib
+        for g in (rec.graph, getattr(rec, "graph_io", None)):
+            if g is not None:
+                lib.vaicu_graph_destroy(g)
+        rec.graph = rec.graph_io = None
+        for pool in rec.loans.values():
+            pool.close()
+        for p in rec.pinned:
+            lib.vaicu_host_free_pinned(p)
+        del rec.pinned[:]
+        seen_buffers = set()
+        for t in list(rec.input_tensors.values()) + rec.keep:
+            b = t.buffer
+            if isinstance(b, (DeviceBuffer, GuardedBuffer)) and id(b) not in seen_buffers and b.ptr is not None:
+                seen_buffers.add(id(b))
+                self.pool.release(b)
+            t.buffer = None
 
     def __del__(self):
         try:
