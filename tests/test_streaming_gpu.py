@@ -39,8 +39,9 @@ def test_streaming_plain(M, K, N, dt, device):
 @pytest.mark.parametrize("w_dtype", ["bf16", "f16"])
 def test_streaming_gate(M, K, H, w_dtype, device):
     x, w, b, _ = _draw(M, K, 2 * H, residual=False)
-    got, want, _ = run_linear(x, w, b, w_dtype=w_dtype, epilogue="SILU", gate_fuse=True)
-    assert_close(got, want, (1e-4, 1e-5), f"gate {M}x{K}x{H} {w_dtype}")
+    for ep in ("SILU", "GELU_TANH"):
+        got, want, _ = run_linear(x, w, b, w_dtype=w_dtype, epilogue=ep, gate_fuse=True)
+        assert_close(got, want, (1e-4, 1e-5), f"gate {ep} {M}x{K}x{H} {w_dtype}")
 
 
 @pytest.mark.parametrize("M", [1, 3, 4, 8])
@@ -137,7 +138,7 @@ def test_streaming_argmax(M, N, device):
 
 def test_streaming_epilogues_and_orders(device):
     x, w, b, r = _draw(7, 776, 333)
-    for M in (2, 7):
+    for M in (1, 2, 7):
         for ep in Epilogue:
             got, want, _ = run_linear(x[:M].copy(), w, b, r[:M].copy(), w_dtype="bf16", epilogue=ep.name,
                                       residual_order="BEFORE_EPILOGUE", scalar_scale=0.25)
