@@ -570,9 +570,9 @@ int build_plan(vaicu_device* dev, const vaicu_linear_desc* desc, const vaicu_lin
     if (kernel == 0) {
         // Few rows: the weight-streaming kernel (vAi useSlabPath takes M <= 8,
         // linear.h:320).  Measured on B200 the FMA kernel stops being memory-bound past
-        // M = 4 (shared-memory reads of the activations), while the swapped tensor-core
-        // kernel streams weights at full rate for any M, so M = 5..8 go there when the
-        // operands allow it.
+        // M = 4 (shared-memory reads of the activations), while the tensor-core kernels
+        // stream weights at full rate for any M, so M = 5..8 go there when the operands
+        // allow it: to skinny_stream_kernel, or to the swapped kernel where that is faster.
         if (d.M <= 4u || (d.M <= 8u && !tc_eligible(d))) kernel = VAICU_KERNEL_GEMV;
         else if (tc_eligible(d)) kernel = d.M <= 128u ? VAICU_KERNEL_TC_SKINNY : VAICU_KERNEL_TC_GEMM;
         else kernel = VAICU_KERNEL_FMA_TILE;

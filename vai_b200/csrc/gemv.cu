@@ -12,8 +12,8 @@
 //   * K is split over `k_warps` warps of a block when N alone cannot fill
 //     148 SMs; the fold goes through shared memory, no global scratch;
 //   * blocks are persistent over row groups (grid sized to the SM count).
-// One row of up to 200 MB of weights takes the streaming form (gemv_stream.cu); this one keeps larger layers, 2 to 8 rows,
-// K beyond 16384, and every geometry that a caller chooses.
+// Most layers of one row take the streaming form (gemv_stream.cu, choose_gemv_stream); this one keeps those above 140 MB, short K
+// over many rows, K beyond 16384 (8192 in fp32), 2 to 8 rows, and every geometry that a caller chooses.
 #include "common.cuh"
 
 namespace vaicu {
@@ -583,8 +583,9 @@ GemvConfig choose_gemv(const LinearArgs& a, int sm_count, bool ptrs_aligned16, c
     // M = 1 comes in two depths: U = 2 k-steps in flight at 3 blocks per SM (96 KB per SM), or U = 4 at
     // 2 blocks per SM (128 KB per SM).  A layer whose weights the resident blocks request in one trip at
     // U = 2 (14.5 MB on 148 SMs) gains nothing from the deeper form and loses resident slots to it; a larger
-    // layer is bound by the bytes in flight (measured in the recorded Llama-3.2-1B step: gate|value and down
-    // at U = 4 take 9 us off 529, the lm_head is unchanged, o at U = 4 adds 11 us).
+    // layer is bound by the bytes in flight (measured in a recorded Llama-3.2-1B step on this form alone: gate|value
+    // and down at U = 4 took 9 us off 529, the lm_head was unchanged, o at U = 4 added 11 us).  The streaming form has
+    // since taken most of both kinds; U = 2 keeps short K (200 x 9000), U = 4 what is above 140 MB.
     const uint64_t one_trip = (uint64_t)sm_count * 3u * (uint64_t)kThreads * 2u * 4u * 16u;
     const uint64_t weight_bytes = (uint64_t)a.N * a.K * (a.w_dtype == VAICU_DTYPE_F32 ? 4u : 2u);
     c.unroll = (a.M == 1u && weight_bytes > one_trip) ? 4 : 2;

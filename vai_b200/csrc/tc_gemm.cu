@@ -10,9 +10,9 @@
 // Structure (one persistent CTA per SM, 384 threads):
 //   warps 0, 10, 11  one lane of each, k-block by k-block in turn, issues TMA loads (cp.async.bulk.tensor, 128-byte swizzle)
 //             into a ring of shared-memory stages, signalled through mbarriers;
-//   warp 1    allocates tensor memory; one lane issues tcgen05.mma
+//   warp 1    allocates tensor memory; one elected lane issues tcgen05.mma
 //             (cta_group::1, M = 128, N = bn, K = 16) and commits each stage back
-//             to the producer and each finished tile to the epilogue;
+//             to the producers and each finished tile to the epilogue;
 //   warps 2-9 read the accumulator with tcgen05.ld (a pair of warps owns 32 TMEM
 //             lanes), apply the epilogue and store.  Two accumulator buffers let
 //             the epilogue of tile i overlap the main loop of tile i+1.
@@ -639,7 +639,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint64_t* empty_bar = full_bar + stages;
     uint64_t* acc_full = empty_bar + stages;      // [2]
     uint64_t* acc_empty = acc_full + 2;           // [2]
-    uint64_t* fold_in = acc_empty + 2;            // split-K fold: the four epilogue warps have written their partials
+    uint64_t* fold_in = acc_empty + 2;            // split-K fold: the epilogue warps have written their partials
     uint64_t* fold_out = fold_in + 1;             // ... and the ticket for this tile has been drawn
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(fold_out + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -1093,12 +1093,12 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar)
 // tcgen05.mma.cta_group::2: each CTA stages its 128 rows of A and HALF of the weights'
 // tile, so shared-memory traffic per MMA cycle halves against the single-CTA kernel
 // and both accumulator buffers (2 x 256 columns) stay available for overlap.
-//   warp 0  (both CTAs) TMA producer for this CTA's boxes; completion bytes of both CTAs
+//   warps 0, 10, 11 (both CTAs) TMA producers, in turn, for this CTA's boxes; completion bytes of both CTAs
 //           are counted on the leader's "full" barrier;
-//   warp 1  allocates tensor memory in both CTAs; in the leader (cluster rank 0) one
-//           lane issues the MMAs and commits to the barriers of both CTAs;
-//   warps 2-5 (both CTAs) epilogue over this CTA's 128 rows; they release an accumulator
-//           by arriving on the leader's barrier.
+//   warp 1  allocates tensor memory in both CTAs; in the leader (cluster rank 0) an
+//           elected lane issues the MMAs and commits to the barriers of both CTAs;
+//   warps 2-9 (both CTAs) epilogue over this CTA's 128 rows, two warps per 32 rows, half of the
+//           tile's columns each; they release an accumulator by arriving on the leader's barrier.
 // With GATE the leader's half of B holds the gate rows and the peer's the value rows.
 // ODD: finished fp32 rows that begin at any element (an odd width, an unaligned view) are staged too.  An instance of its own:
 // with both ways of storing in one, 1024 rows of a GPT-2-small model took 1.5 % longer, a 333-row block 0.8 %.
